@@ -182,6 +182,7 @@ static __device__ unsigned long long g_wait_limit_ns = kBarrierTimeoutNs;
     }
 int set_wait_limit_projection(unsigned long long ns);
 int set_wait_limit_mgpcg(unsigned long long ns);
+int set_wait_limit_cgres(unsigned long long ns);
 
 __device__ __forceinline__ unsigned long long global_ns()
 {

@@ -118,9 +118,13 @@ extern "C" int ffr_poisson_solve_noalloc(int nx, int ny, int nz, const double *d
     a.out_res = out_res; a.out_iters = out_it; a.out_flags = out_fl;
     const unsigned blocks = (unsigned)std::max<long long>(
         1, std::min<long long>(std::min<long long>(cg_block_cap(), kNoAllocMaxBlocks), (n + 255) / 256));
-    void *args[] = {(void *)&a};
-    FFR_CUDA(cudaLaunchCooperativeKernel((void *)k_cg, dim3(blocks), dim3(256), args, 0, st));
-    count_launch(1);
+    bool taken = false;
+    if (blocks == cdiv(n, 256) && (rc = launch_cg_resident(a, st, &taken))) return rc;
+    if (!taken) {
+        void *args[] = {(void *)&a};
+        FFR_CUDA(cudaLaunchCooperativeKernel((void *)k_cg, dim3(blocks), dim3(256), args, 0, st));
+        count_launch(1);
+    }
     double res = 0.0;
     int it = 0, fl = 0;
     FFR_CUDA(cudaMemcpyAsync(&res, out_res, 8, cudaMemcpyDeviceToHost, st));

@@ -1181,6 +1181,7 @@ extern "C" int ffr_set_device_wait_limit(double seconds)
         seconds == 0.0 ? kBarrierTimeoutNs : (unsigned long long)(seconds * 1e9 + 0.5);
     int rc = set_wait_limit_projection(ns);
     if (!rc) rc = set_wait_limit_mgpcg(ns);
+    if (!rc) rc = set_wait_limit_cgres(ns);
     return rc;
 }
 
@@ -1367,6 +1368,12 @@ namespace {
 
 int launch_cg(const CGArgs &a, unsigned blocks, cudaStream_t s)
 {
+    // one cell per thread: the on-chip form (the same sums in the same order)
+    if (blocks == cdiv(a.R.n, kThreads)) {
+        bool taken = false;
+        const int rc = launch_cg_resident(a, s, &taken);
+        if (rc || taken) return rc;
+    }
     FFR_CUDA(cudaMemsetAsync(a.gs, 0, sizeof(GridSync), s));
     void *args[] = {(void *)&a};
     FFR_CUDA(cudaLaunchCooperativeKernel((void *)k_cg, dim3(blocks), dim3(kThreads), args, 0, s));

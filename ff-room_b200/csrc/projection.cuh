@@ -77,5 +77,10 @@ struct CGArgs {
 // (projection.cu).
 __global__ void __launch_bounds__(256) k_cg(CGArgs A);
 unsigned cg_block_cap();
+// The same solve with its vectors on chip (cgres.cu), for a room that k_cg's
+// natural grid gives one cell per thread.  *taken = false (nothing launched)
+// when the room does not fit.  A.da and A.db (slices of one allocation, da
+// first) and A.ad are its scratch.
+int launch_cg_resident(const CGArgs &a, cudaStream_t s, bool *taken);
 
 }  // namespace ffr
