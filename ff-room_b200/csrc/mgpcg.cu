@@ -619,6 +619,12 @@ __device__ __forceinline__ double face_rhs(const PCGArgs &A, int c, int i, int j
     return A.rhs_factor * div;
 }
 
+}  // namespace ffr
+
+#include "mgonchip.cuh"
+
+namespace ffr {
+
 // Synchronisation groups of the preconditioned solve.
 //  GridGroup    - every block of a cooperative launch (one room on the whole GPU)
 //  ClusterGroup - the blocks of one thread-block cluster (one room on 1-16 SMs;
@@ -1058,19 +1064,35 @@ __device__ __forceinline__ void pass_backsub(const PCGArgs &A, int start, int st
     }
 }
 
+// A block's copy of its room's arguments.
+__device__ __forceinline__ void load_args(PCGArgs &dst, const PCGArgs *src)
+{
+    static_assert(sizeof(PCGArgs) % 8 == 0, "PCGArgs copy in 8-byte words");
+    const unsigned long long *s = reinterpret_cast<const unsigned long long *>(src);
+    unsigned long long *d = reinterpret_cast<unsigned long long *>(&dst);
+    for (int i = threadIdx.x; i < (int)(sizeof(PCGArgs) / 8); i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+}
+
 // Threads per block of the one-cluster schedule: a cluster of at most 16
 // blocks must still hold enough warps per SM to hide memory latency.
 constexpr int kClusterThreads = 512;
 
 // The whole solve on the blocks of group G (a cooperative grid or one
 // thread-block cluster).
-template <class G>
+// ONCHIP: the V-cycle from level A.Q.lo down runs in the cluster's shared
+// memory (mgonchip.cuh), the levels above it and the FP64 passes in global
+// memory.
+template <class G, bool ONCHIP>
 __device__ __forceinline__ void pcg_body(const PCGArgs &A)
 {
     __shared__ double sh[32];
     if (A.st && A.st->halt) return;
     const MGDev &M = A.M;
     G::init();
+    __shared__ OcLevels oc;
+    if constexpr (ONCHIP) oc_setup(A, A.Q, G::rank(), oc);
+    const int lo = ONCHIP ? A.Q.lo : min(M.nlev_grid, M.nlev - 1);   // first level not swept by the group
     const int t0 = G::rank() * blockDim.x + threadIdx.x, nth = G::size() * blockDim.x;
     int flags = 0, iters = 0;
     double res = 0.0;
@@ -1086,7 +1108,7 @@ __device__ __forceinline__ void pcg_body(const PCGArgs &A)
         bool pending = false;
         for (int it = 0;; it++) {
             // ---- preconditioner: V-cycle from the red sweep already in z
-            for (int l = 0; l < M.nlev_grid && l < M.nlev - 1; l++) {
+            for (int l = 0; l < lo; l++) {
                 smooth_color<false>(A, M.lv, M.nlev, l, 1, t0, nth);
                 if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
                 for (int sw = 1; sw < level_sweeps(l); sw++) {
@@ -1098,11 +1120,14 @@ __device__ __forceinline__ void pcg_body(const PCGArgs &A)
                 restrict_level(A, M.lv, l, t0, nth);
                 if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
             }
-            if (M.nlev_grid < M.nlev) {
+            if constexpr (ONCHIP) {
+                oc_vcycle<true>(A, A.Q, G::rank(), oc);
+                if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
+            } else if (M.nlev_grid < M.nlev) {
                 if (G::rank() == 0) block_vcycle(A, M.nlev_grid);
                 if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
             }
-            for (int l = min(M.nlev_grid, M.nlev - 1) - 1; l >= 1; l--) {
+            for (int l = lo - 1; l >= 1; l--) {
                 smooth_color<true>(A, M.lv, M.nlev, l, 1, t0, nth);
                 if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
                 smooth_color<false>(A, M.lv, M.nlev, l, 0, t0, nth);
@@ -1114,7 +1139,7 @@ __device__ __forceinline__ void pcg_body(const PCGArgs &A)
                     if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
                 }
             }
-            if (M.nlev_grid >= 1 && M.nlev > 1) {
+            if (lo >= 1 && M.nlev > 1) {
                 smooth_color<true>(A, M.lv, M.nlev, 0, 1, t0, nth);
                 if (!G::sync(A)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
                 // the further sweeps; the last red half is the r.z pass's
@@ -1173,25 +1198,29 @@ finish:
     }
 }
 
-template <class G, int NT = 256>
+template <class G, int NT = 256, bool ONCHIP = false>
 __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 1) k_pcg(PCGArgs A)
 {
-    pcg_body<G>(A);
+    if constexpr (ONCHIP) {
+        __shared__ __align__(16) PCGArgs S;
+        load_args(S, &A);
+        pcg_body<G, ONCHIP>(S);
+    } else {
+        pcg_body<G, ONCHIP>(A);
+    }
 }
 
 // Batched rooms, one thread-block cluster per room: cluster c (blocks
 // c*ctas .. c*ctas + ctas - 1) runs the whole solve of room order[c], exactly as
 // that room's own one-cluster launch (k_pcg<ClusterGroup>) does, so many
 // rooms' solves run side by side in one launch with no host pacing.
+template <bool ONCHIP>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_bpcg_cluster(BatchDev D, const int *order, int ctas)
 {
     __shared__ __align__(16) PCGArgs A;
     const int r = order[blockIdx.x / (unsigned)ctas];
-    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(D.args + r);
-    unsigned long long *dst = reinterpret_cast<unsigned long long *>(&A);
-    for (int i = threadIdx.x; i < (int)(sizeof(PCGArgs) / 8); i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
-    pcg_body<ClusterGroup>(A);
+    load_args(A, D.args + r);
+    pcg_body<ClusterGroup, ONCHIP>(A);
 }
 
 // ================================================================ split
@@ -1435,6 +1464,18 @@ __global__ void __launch_bounds__(kMidThreads, 1) k_sp_mid(PCGArgs A, const Spli
     sp_mid_body(A, mid);
 }
 
+// The same levels (A.Q.lo on) in the cluster's shared memory.
+__global__ void __launch_bounds__(kMidThreads, 1) k_sp_mid_onchip(PCGArgs A, const SplitState *ss)
+{
+    if (ss->done) return;
+    __shared__ __align__(16) PCGArgs S;
+    load_args(S, &A);
+    const int rank = (int)cooperative_groups::this_cluster().block_rank();
+    __shared__ OcLevels oc;
+    oc_setup(S, S.Q, rank, oc);
+    oc_vcycle<false>(S, S.Q, rank, oc);
+}
+
 __global__ void __launch_bounds__(256) k_sp_redpost(PCGArgs A, SplitState *ss)
 {
     if (ss->done) return;
@@ -1479,15 +1520,6 @@ __global__ void __launch_bounds__(256) k_sp_backsub(PCGArgs A, const SplitState 
 // m.first[r + 1] - 1, as many as its one-room launch has, so every room
 // computes exactly what its own launch would.  Each block copies its room's
 // arguments to shared memory first.
-
-__device__ __forceinline__ void load_args(PCGArgs &dst, const PCGArgs *src)
-{
-    static_assert(sizeof(PCGArgs) % 8 == 0, "PCGArgs copy in 8-byte words");
-    const unsigned long long *s = reinterpret_cast<const unsigned long long *>(src);
-    unsigned long long *d = reinterpret_cast<unsigned long long *>(&dst);
-    for (int i = threadIdx.x; i < (int)(sizeof(PCGArgs) / 8); i += blockDim.x) d[i] = s[i];
-    __syncthreads();
-}
 
 __global__ void __launch_bounds__(256) k_bsp_extrapolate(BatchDev D, BMap m)
 {
@@ -1756,18 +1788,88 @@ unsigned pcg_max_blocks()
     return cap;
 }
 
-int launch_pcg_cluster(const PCGArgs &a, cudaStream_t s, int ctas)
+namespace {
+
+int plane_pairs(const MGLevel &L) { return L.ny * ((L.nz + 1) >> 1); }
+
+// Shared memory left to the on-chip V-cycle beside a kernel's static arrays.
+constexpr size_t kOnchipBytes = 220 * 1024;
+
+template <class F> int allow_cluster(F *fn, size_t smem)
 {
-    static bool attr_set = false;
-    if (!attr_set) {
-        FFR_CUDA(cudaFuncSetAttribute(k_pcg<ClusterGroup, kClusterThreads>,
-                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        attr_set = true;
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (smem) FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOnchipBytes));
+    return FFR_OK;
+}
+
+}  // namespace
+
+// The finest level that fits: up to about 150 k cells on 16 blocks that is
+// level 0.  Per iteration with 16 blocks, the V-cycle in global memory and on
+// chip: 15 k cells (8 blocks) 103 -> 80 us, 52 k 142 -> 110, 92 k 159 -> 124,
+// 192 k (from level 1 on) 224 -> 201; the levels of at most 32 k cells below a
+// split solve (k_sp_mid) 70 -> 40 us.
+bool plan_onchip(const MGDev &M, int ctas, int lo_min, size_t bytes, OnchipPlan &out)
+{
+    // (a hierarchy that could not be coarsened to a block-sized level has no
+    // coarsest solve in the other forms, and no plan here)
+    const bool coarsened = M.nlev > 1 && M.nlev_grid < M.nlev;
+    for (int lo = lo_min; lo < M.nlev && coarsened; lo++) {
+        OnchipPlan Q{};
+        Q.lo = lo;
+        Q.fb = std::max(lo, 1);
+        while (Q.fb < M.nlev - 1 && M.lv[Q.fb].n > kOcBlockCells) Q.fb++;
+        // a block's planes on every split level: halved with the axis, so a
+        // coarse plane's children are in the same block
+        int align = 1;
+        for (int l = lo; l + 1 < Q.fb; l++) align <<= M.lv[l].sx;
+        const int want = (M.lv[lo].nx + ctas - 1) / ctas;
+        int P = (want + align - 1) / align * align;
+        Q.blocks = Q.fb > lo ? (M.lv[lo].nx + P - 1) / P : 1;
+        long long floats = 0, red = 0;
+        for (int l = lo; l < M.nlev; l++) {
+            const long long rp = plane_pairs(M.lv[l]);
+            if (l >= Q.fb) P = M.lv[l].nx;
+            Q.planes[l] = P;
+            Q.off[l] = (int)floats;
+            Q.mag_rp[l] = 0xFFFFFFFFu / (unsigned)rp + 1u;
+            Q.mag_pk[l] = 0xFFFFFFFFu / (unsigned)((M.lv[l].nz + 1) >> 1) + 1u;
+            floats += rp * (2 * (P + 2) + 4 * P + (l == 0 ? P : 6 * (P + 1)));
+            Q.off_flag[l] = (int)floats;
+            floats += (rp * P + 3) / 4;
+            if (l + 1 != Q.fb) red = std::max(red, rp * P);
+            if (l + 1 == Q.fb) {
+                const MGLevel &B = M.lv[Q.fb];
+                Q.off_res = (int)floats;
+                floats += (long long)M.lv[l].nx * rp;
+                Q.off_par = (int)floats;
+                floats += 2ll * ((P >> M.lv[l].sx) + 3) * plane_pairs(B);
+            }
+            if (l + 1 < Q.fb) P >>= M.lv[l].sx;
+            if (4 * floats > (long long)bytes) break;
+        }
+        Q.off_red = (int)floats;
+        floats += red;
+        Q.floats = (int)floats;
+        if (4 * floats <= (long long)bytes) {
+            out = Q;
+            return true;
+        }
     }
+    out = OnchipPlan{};
+    return false;
+}
+
+int launch_pcg_cluster(const PCGArgs &a0, cudaStream_t s, int ctas)
+{
+    PCGArgs a = a0;
+    const bool onchip = plan_onchip(a.M, ctas, 0, kOnchipBytes, a.Q);
+    auto *fn = onchip ? k_pcg<ClusterGroup, kClusterThreads, true> : k_pcg<ClusterGroup, kClusterThreads, false>;
+    if (int rc = allow_cluster(fn, onchip)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = onchip ? 4 * (size_t)a.Q.floats : 0;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1776,7 +1878,7 @@ int launch_pcg_cluster(const PCGArgs &a, cudaStream_t s, int ctas)
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FFR_CUDA(cudaLaunchKernelEx(&cfg, k_pcg<ClusterGroup, kClusterThreads>, a));
+    FFR_CUDA(cudaLaunchKernelEx(&cfg, fn, a));
     count_launch(1);
     return FFR_OK;
 }
@@ -1829,6 +1931,7 @@ int mid_cluster_ctas()
     static int ctas = 0;
     if (ctas) return ctas;
     cudaFuncSetAttribute(k_sp_mid, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (allow_cluster(k_sp_mid_onchip, kOnchipBytes)) cudaGetLastError();
     for (int want : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)want);
@@ -1905,7 +2008,14 @@ int split_iteration(const PCGArgs &a, SplitState *ss, cudaStream_t bs, cudaGraph
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            cudaError_t e = cudaLaunchKernelEx(&cfg, k_sp_mid, a, (const SplitState *)ss, M.nlev_mid);
+            PCGArgs am = a;
+            cudaError_t e;
+            if (plan_onchip(M, ctas, M.nlev_mid, kOnchipBytes, am.Q) && am.Q.lo == M.nlev_mid) {
+                cfg.dynamicSmemBytes = 4 * (size_t)am.Q.floats;
+                e = cudaLaunchKernelEx(&cfg, k_sp_mid_onchip, am, (const SplitState *)ss);
+            } else {
+                e = cudaLaunchKernelEx(&cfg, k_sp_mid, a, (const SplitState *)ss, M.nlev_mid);
+            }
             if (e != cudaSuccess && rc == FFR_OK) rc = cuda_fail(e, "cudaLaunchKernelEx(k_sp_mid)");
             chk();
         }
@@ -2114,10 +2224,19 @@ unsigned build_map(std::vector<int> &room, std::vector<int> &first, const std::v
 
 }  // namespace
 
-int batch_split_build(BatchSplit &B, const std::vector<PCGArgs> &args, const std::vector<void *> &ss)
+int batch_split_build(BatchSplit &B, std::vector<PCGArgs> &args, const std::vector<void *> &ss, int ctas)
 {
     const int n = (int)args.size();
     B.nrooms = n;
+    B.cluster_floats = 0;
+    if (ctas > 0) {
+        bool all = true;
+        for (PCGArgs &a : args) {
+            all = plan_onchip(a.M, ctas, 0, kOnchipBytes, a.Q) && all;
+            B.cluster_floats = std::max(B.cluster_floats, a.Q.floats);
+        }
+        if (!all) B.cluster_floats = 0;
+    }
     if (n == 0) return FFR_OK;
     std::vector<RoomShape> sh(n);
     int nlev = 0;
@@ -2325,16 +2444,15 @@ int batch_split_solve(BatchSplit &B, cudaStream_t s, int max_iter)
 int launch_batch_cluster(BatchSplit &B, cudaStream_t s, int ctas)
 {
     if (B.nrooms == 0) return FFR_OK;
-    static bool attr_set = false;
-    if (!attr_set) {
-        FFR_CUDA(cudaFuncSetAttribute(k_bpcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        attr_set = true;
-    }
+    const bool onchip = B.cluster_floats > 0;
+    auto *fn = onchip ? k_bpcg_cluster<true> : k_bpcg_cluster<false>;
+    if (int rc = allow_cluster(fn, onchip)) return rc;
     k_bsp_extrapolate<<<B.nb_cells0, 256, 0, s>>>(B.D, B.cells0);
     FFR_LAUNCHED(1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(B.nrooms * ctas));
     cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = 4 * (size_t)B.cluster_floats;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2343,7 +2461,7 @@ int launch_batch_cluster(BatchSplit &B, cudaStream_t s, int ctas)
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FFR_CUDA(cudaLaunchKernelEx(&cfg, k_bpcg_cluster, B.D, B.cluster_order, ctas));
+    FFR_CUDA(cudaLaunchKernelEx(&cfg, fn, B.D, B.cluster_order, ctas));
     count_launch(1);
     return FFR_OK;
 }

@@ -57,6 +57,25 @@ struct MGDev {
     float *r32;           // FP32 copy of the scaled CG residual (level-0 rhs)
 };
 
+// How one thread-block cluster keeps the V-cycle from level lo down in shared
+// memory (mgonchip.cuh): levels lo .. fb-1 split over its blocks by whole
+// i-planes, the levels from fb on in block 0.
+constexpr int kOcBlockCells = 2048;
+struct OnchipPlan {
+    int lo, fb;               // lo == 0 and fb == 0: no plan
+    int blocks;               // blocks that hold planes
+    int planes[kMaxLevels];   // planes of a block
+    int off[kMaxLevels], off_flag[kMaxLevels];   // a level's arrays and bytes (in floats)
+    unsigned mag_rp[kMaxLevels], mag_pk[kMaxLevels];   // reciprocals of its pairs per plane and per row
+    int off_res, off_par;     // red residuals of level fb-1 (block 0), copied parents
+    int off_red;              // red residuals of a block's own planes
+    int floats;
+};
+// The plan of a hierarchy for a cluster of `ctas` blocks: from the finest
+// level >= lo_min on that fits `bytes` of shared memory per block.  False
+// (and no plan) when none does.
+bool plan_onchip(const MGDev &M, int ctas, int lo_min, size_t bytes, OnchipPlan &out);
+
 // Host side: the level sizes of a room's hierarchy.
 struct MGHost {
     std::vector<int> nx, ny, nz;
@@ -93,6 +112,7 @@ struct PCGArgs {
     double *out_res;
     int *out_iters;
     int *out_flags;
+    OnchipPlan Q;                  // one-cluster schedules
 };
 // Warm start of the next solve, queued before it: x0 = x + theta (x - xprev)
 // (x the previous step's solution, xprev the one before; theta 0 on a
@@ -174,6 +194,7 @@ struct BatchSplit {
     unsigned nb_post0 = 0;
     const int *mid_rooms = nullptr;   // rooms with levels small enough for one block
     const int *cluster_order = nullptr;   // rooms largest first (one-cluster-per-room launch)
+    int cluster_floats = 0;           // on-chip V-cycle: the largest room's shared memory; 0: not every room has a plan
     int nmid = 0;
     void *dev = nullptr;              // device allocation holding all tables
     size_t cap = 0;                   // its size (reused while large enough)
@@ -185,7 +206,8 @@ struct BatchSplit {
 // copies; device pointers inside) and device split states.  The device
 // buffer of an earlier build is reused when large enough; no launch of an
 // earlier build may still be running.
-int batch_split_build(BatchSplit &B, const std::vector<PCGArgs> &args, const std::vector<void *> &ss);
+// ctas: blocks per room of the one-cluster-per-room launch (0: not used).
+int batch_split_build(BatchSplit &B, std::vector<PCGArgs> &args, const std::vector<void *> &ss, int ctas);
 void batch_split_release(BatchSplit &B);
 // The split solve of every room of the batch, host-paced like
 // launch_split_pcg: iterations are queued in batches until no room is

@@ -2327,7 +2327,7 @@ int ffr_batch_set_rooms(ffr_batch *b, ffr_fluid *const *rooms, int nrooms)
     b->open = reinterpret_cast<const OpenItem *>(put(oitems.data(), sizeof(OpenItem) * oitems.size()));
     b->heat = reinterpret_cast<const HeatItem *>(put(hitems.data(), sizeof(HeatItem) * hitems.size()));
     FFR_CUDA(cudaMemcpy(b->dev, host.data(), bytes, cudaMemcpyHostToDevice));
-    const int rc = batch_split_build(b->split, pa, ss);
+    const int rc = batch_split_build(b->split, pa, ss, b->cluster_ctas);
     if (rc == FFR_OK) b->stale = false;
     return rc;
 }
