@@ -15,7 +15,8 @@
 //   3. takes the moments (the reference's extract_macroscopic input) and
 //      writes the cell velocity and p = rho*cs^2;
 //   4. applies the next step's inflow BC / BGK collision and stores f*.
-// A second kernel forms the face velocities, max |du| and max |div|.
+// A second kernel forms the face velocities, max |du| and max |div|; its last
+// block closes the step.
 //
 // Storage modes: FP64 (the reference arithmetic), FP32 and FP16.  The
 // narrow modes store the shifted populations g_q = f_q - w_q (the "DDF
@@ -114,16 +115,40 @@ __device__ __forceinline__ float geq32(int q, float drho, float ux, float uy, fl
 template <int MODE> struct Store;
 template <> struct Store<0> {
     using T = double;
+    __device__ static void ld2(const double *p, double &a, double &b)
+    {
+        const double2 v = *reinterpret_cast<const double2 *>(p);
+        a = v.x;
+        b = v.y;
+    }
+    __device__ static void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
     __device__ static double ld(const double *p) { return *p; }
     __device__ static void st(double *p, double v) { *p = v; }
 };
 template <> struct Store<1> {
     using T = float;
+    __device__ static void ld2(const float *p, float &a, float &b)
+    {
+        const float2 v = *reinterpret_cast<const float2 *>(p);
+        a = v.x;
+        b = v.y;
+    }
+    __device__ static void st2(float *p, float a, float b) { *reinterpret_cast<float2 *>(p) = make_float2(a, b); }
     __device__ static float ld(const float *p) { return *p; }
     __device__ static void st(float *p, float v) { *p = v; }
 };
 template <> struct Store<2> {
     using T = __half;
+    __device__ static void ld2(const __half *p, float &a, float &b)
+    {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(p));
+        a = v.x;
+        b = v.y;
+    }
+    __device__ static void st2(__half *p, float a, float b)
+    {
+        *reinterpret_cast<__half2 *>(p) = __halves2half2(__float2half_rn(a), __float2half_rn(b));
+    }
     __device__ static float ld(const __half *p) { return __half2float(*p); }
     __device__ static void st(__half *p, float v) { *p = __float2half_rn(v); }
 };
@@ -134,6 +159,7 @@ enum : uint8_t { LF_OPEN = 4,    // all 18 neighbours in the domain and not SOLI
 
 struct LbmDev {
     int nx, ny, nz, n, nu, nv, nw;
+    int np;                     // populations per direction: f_q of cell c is f[q * np + c]
     const uint8_t *ct;          // cell types
     const uint8_t *fl;          // cell type | LF_* flags
     const uint32_t *blk;        // bit q: x + e_q outside the room or SOLID (non-open cells)
@@ -151,149 +177,373 @@ struct LbmState {
     int step, halt, stop_on_converge, par;
     unsigned long long dmax_bits, div_bits;
     int ring_slot, flags;
+    unsigned ticket, pad;
 };
-
-__device__ __forceinline__ int find_src(const LbmDev &L, int c)
-{
-    int lo = 0, hi = L.nremap - 1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const int d = L.remap_dst[mid];
-        if (d == c) return L.remap_src[mid];
-        if (d < c) lo = mid + 1; else hi = mid - 1;
-    }
-    return c;
-}
 
 // Cell-centred velocity between the step and face kernels: FP64 with FP64
 // populations, FP32 with the narrow storage modes (their collision is FP32).
 template <int MODE> using CellVel = typename std::conditional<MODE == 0, double, float>::type;
 
-// One fused step; see the file comment.  fa = f* of this step, fb = f* of
-// the next, cu/cv/cw = cell-centred velocity (m/s), p = rho*cs^2.
+// Two FP32 values, one per cell of a pair, in the packed arithmetic of sm_100
+// (each half rounded as the scalar operation rounds it).
+struct F2 {
+    unsigned long long v;
+    __device__ __forceinline__ static F2 of(float a, float b)
+    {
+        F2 r;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+        return r;
+    }
+    __device__ __forceinline__ static F2 all(float a) { return of(a, a); }
+    __device__ __forceinline__ void get(float &a, float &b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+};
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// a - b (one rounding, like the scalar subtraction)
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, F2::all(-1.0f), a); }
+
+// Moments and BGK collision of a pair of cells in shifted FP32 populations:
+// add_moments and geq32 (fused as the compiler fuses those), the terms that a
+// direction and its reverse share formed once.  Returns the velocities and
+// drho; f becomes the post-collision populations.
+// (itau 0 leaves a cell's populations as they are.)
+__device__ __forceinline__ void collide_pair(float (&f0)[19], float (&f1)[19], float itau0, float itau1, float (&u0)[3],
+                                             float (&u1)[3], float &drho0, float &drho1)
+{
+    F2 f[19];
+#pragma unroll
+    for (int q = 0; q < 19; q++) f[q] = F2::of(f0[q], f1[q]);
+    F2 d = f[0], j[3] = {F2::all(0.0f), F2::all(0.0f), F2::all(0.0f)};
+#pragma unroll
+    for (int q = 1; q < 19; q++) {
+        d = f2_add(d, f[q]);
+        const int e[3] = {c_ex(q), c_ey(q), c_ez(q)};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (e[a] > 0) j[a] = f2_add(j[a], f[q]);
+            else if (e[a] < 0) j[a] = f2_sub(j[a], f[q]);
+        }
+    }
+    d.get(drho0, drho1);
+    const float rho0 = 1.0f + drho0, rho1 = 1.0f + drho1;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        j[a].get(u0[a], u1[a]);
+        if (rho0 > 1e-14f) u0[a] /= rho0;
+        if (rho1 > 1e-14f) u1[a] /= rho1;
+    }
+    const F2 u[3] = {F2::of(u0[0], u1[0]), F2::of(u0[1], u1[1]), F2::of(u0[2], u1[2])};
+    const F2 rho = F2::of(rho0, rho1), nt = F2::of(-itau0, -itau1), c15 = F2::all(-1.5f), c45 = F2::all(4.5f),
+             p3 = F2::all(3.0f), m3 = F2::all(-3.0f);
+    const F2 usq = f2_fma(u[2], u[2], f2_fma(u[0], u[0], f2_mul(u[1], u[1])));
+    // fq + itau (w (drho + rho k) - fq), the two signs folded into the factors
+    auto relax = [&](int q, F2 k) {
+        const F2 y = f2_fma(rho, k, d);
+        f[q] = f2_fma(nt, f2_fma(F2::all(-(float)lbm_w(q)), y, f[q]), f[q]);
+    };
+    relax(0, f2_mul(c15, usq));
+#pragma unroll
+    for (int q = 1; q < 19; q++) {
+        const int r = c_rev(q);
+        if (r < q) continue;
+        // e_q . u; the reverse direction's is its negative
+        F2 eu = F2::all(0.0f);
+        bool any = false;
+        const int e[3] = {c_ex(q), c_ey(q), c_ez(q)};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (e[a] > 0) { eu = any ? f2_add(eu, u[a]) : u[a]; any = true; }
+            else if (e[a] < 0) { eu = any ? f2_sub(eu, u[a]) : f2_mul(u[a], F2::all(-1.0f)); any = true; }
+        }
+        const F2 m = f2_mul(f2_mul(c45, eu), eu);
+        relax(q, f2_fma(c15, usq, f2_fma(p3, eu, m)));
+        relax(r, f2_fma(c15, usq, f2_fma(m3, eu, m)));
+    }
+#pragma unroll
+    for (int q = 0; q < 19; q++) f[q].get(f0[q], f1[q]);
+}
+
+// Blocks of 256 threads per SM the step's registers are cut for (pairs: FP16
+// 64 registers and a few spills, 395 us against 445 with 80 at 15.7 M cells;
+// FP32 80 registers, 498 against 520 with 64).
+template <int MODE, int NV> struct LbmLaunch { static constexpr int blocks = MODE == 0 ? (NV == 1 ? 3 : 2) : (MODE == 1 ? 3 : 4); };
+
+// Whether the distance ex * plane + ey * row + ez is odd (PAR as in k_lbm_step).
+template <int PAR> __host__ __device__ constexpr bool constexpr_parity(int q)
+{
+    return ((PAR == 2 ? c_ex(q) : 0) + (PAR >= 1 ? c_ey(q) : 0) + c_ez(q)) & 1;
+}
+
+// Slots of a cell next to a wall or SOLID (bit q of B: cell + e_q is outside
+// the room or SOLID; fq holds f*_q(x - e_q) for the open directions).  Slot q
+// receives
+//  (a) f*_q(x - e_q) when x - e_q = x + e_{-q} is not blocked;
+//  (b) f*_OPP[q](x) when x's own direction OPP[q] is blocked.
+// OPP of LBMSolver.cpp:27 pairs the diagonals as mirror images (7 <-> 8 is
+// (1,1,0) <-> (-1,1,0)), so (a) and (b) are independent and a slot gets 0, 1
+// or 2 values.
+template <int MODE, class C>
+__device__ __forceinline__ void fix_blocked(const LbmDev &L, const typename Store<MODE>::T *fa, int o, unsigned B,
+                                            C (&fq)[19])
+{
+#pragma unroll
+    for (int q = 0; q < 19; q++) {
+        const int qq = c_opp(q);
+        const bool ina = !((B >> c_rev(q)) & 1u);
+        const bool inb = (B >> qq) & 1u;
+        const C va = fq[q];
+        const C vb = inb ? C(Store<MODE>::ld(fa + ((size_t)qq * L.np + o))) : C(0);
+        if (MODE == 0) {
+            // the reference's zeroed slot plus what arrives
+            fq[q] = ina ? (inb ? va + vb : va) : vb;
+        } else {
+            // shifted storage g = f - w (w_q == w_OPP[q]): two arrivals give
+            // g_a + g_b + w, none gives -w
+            fq[q] = ina ? (inb ? va + vb + C(lbm_w(q)) : va) : (inb ? vb : C(-lbm_w(q)));
+        }
+    }
+}
+
+// The fan equilibrium of an INFLOW cell (shifted FP32 populations).
+__device__ __forceinline__ void inflow32(const LbmDev &L, int o, float (&fq)[19])
+{
+    if (L.fan_of[o] == 255) return;
+    const double *fv = L.fan_lat + 3 * L.fan_of[o];
+#pragma unroll
+    for (int q = 0; q < 19; q++) fq[q] = geq32(q, 0.0f, (float)fv[0], (float)fv[1], (float)fv[2]);
+}
+
+// Moments of one cell's populations and their inflow / collision for the next
+// step: the velocity (m/s), p = rho cs^2 and the post-collision populations.
+template <int MODE, class C>
+__device__ __forceinline__ void collide_cell(const LbmDev &L, int o, unsigned t, C (&fq)[19], C &vx, C &vy, C &vz, double &p)
+{
+    if constexpr (MODE == 0) {
+        double rho = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
+#pragma unroll
+        for (int q = 0; q < 19; q++) add_moments<double>(q, fq[q], rho, ux, uy, uz);
+        if (rho > 1e-14) { ux /= rho; uy /= rho; uz /= rho; }
+        vx = ux * L.l2p; vy = uy * L.l2p; vz = uz * L.l2p;
+        p = rho * (1.0 / 3.0);
+        if (t == CT_INFLOW) {
+            if (L.fan_of[o] != 255) {
+                const double *fv = L.fan_lat + 3 * L.fan_of[o];
+#pragma unroll
+                for (int q = 0; q < 19; q++) fq[q] = feq64(q, 1.0, fv[0], fv[1], fv[2]);
+            }
+        } else {
+            const double itau = 1.0 / L.tau;
+#pragma unroll
+            for (int q = 0; q < 19; q++) {
+                const double fe = feq64(q, rho, ux, uy, uz);
+                fq[q] = fq[q] + itau * (fe - fq[q]);
+            }
+        }
+    } else {
+        float drho = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 19; q++) add_moments<float>(q, fq[q], drho, jx, jy, jz);
+        const float rho = 1.0f + drho;
+        float ux = jx, uy = jy, uz = jz;
+        if (rho > 1e-14f) { ux /= rho; uy /= rho; uz /= rho; }
+        vx = (float)((double)ux * L.l2p);
+        vy = (float)((double)uy * L.l2p);
+        vz = (float)((double)uz * L.l2p);
+        p = (double)rho * (1.0 / 3.0);
+        if (t == CT_INFLOW) {
+            inflow32(L, o, fq);
+        } else {
+            const float itau = (float)(1.0 / L.tau);
+#pragma unroll
+            for (int q = 0; q < 19; q++) {
+                const float ge = geq32(q, drho, ux, uy, uz);
+                fq[q] = fq[q] + itau * (ge - fq[q]);
+            }
+        }
+    }
+}
+
+// The step of the re-mapped OUTFLOW cells i, i + stride, ... of the list: their
+// post-stream populations are those of another cell o (gathered as that cell
+// gathers its own), from there on the cell's own step.
 template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 0 ? 3 : 4)
-    k_lbm_step(LbmDev L, const typename Store<MODE>::T *f0, typename Store<MODE>::T *f1,
-               CellVel<MODE> *__restrict__ cu, CellVel<MODE> *__restrict__ cv, CellVel<MODE> *__restrict__ cw,
-               double *__restrict__ p, const LbmState *st)
+__device__ __forceinline__ void step_remapped(const LbmDev &L, const typename Store<MODE>::T *__restrict__ fa,
+                                              typename Store<MODE>::T *__restrict__ fb, CellVel<MODE> *cu,
+                                              CellVel<MODE> *cv, CellVel<MODE> *cw, double *p, int i, int stride)
 {
     using S = Store<MODE>;
-    using T = typename S::T;
-    if (st->halt) return;
-    const T *__restrict__ fa = st->par ? f1 : f0;
-    T *__restrict__ fb = st->par ? (T *)f0 : f1;
-    const int ny = L.ny, nz = L.nz, n = L.n, plane = ny * nz;
-    // The flags and blocked-direction mask of the next cell are loaded while
-    // this cell's populations are in flight, so each cell waits for one
-    // round trip to memory only.
-    const int c0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    uint8_t fl = 0, fln = 0;
-    unsigned Bc = 0, Bn = 0;
-    // (interior cells have no blocked direction and skip the mask load)
-    if (c0 < n) { fl = L.fl[c0]; Bc = (fl & LF_OPEN) ? 0u : L.blk[c0]; }
-    for (int c = c0; c < n; c += stride, fl = fln, Bc = Bn) {
-        if (c + stride < n) {
-            fln = L.fl[c + stride];
-            Bn = (fln & LF_OPEN) ? 0u : L.blk[c + stride];
-        }
-        const uint8_t t = fl & 3;
-        if (t == CT_SOLID) {
-            cu[c] = 0; cv[c] = 0; cw[c] = 0;
-            continue;
-        }
-        using C = typename std::conditional<MODE == 0, double, float>::type;
+    using C = typename std::conditional<MODE == 0, double, float>::type;
+    const int plane = L.ny * L.nz;
+    for (; i < L.nremap; i += stride) {
+        const int c = L.remap_dst[i], o = L.remap_src[i];
         C fq[19];
-        // x: the cell whose post-stream populations this cell ends with
-        const int o = (fl & LF_REMAP) ? find_src(L, c) : c;
-        if ((fl & LF_REMAP) && L.ct[o] == CT_SOLID) {
+        if (L.ct[o] == CT_SOLID) {
 #pragma unroll
             for (int q = 0; q < 19; q++) fq[q] = MODE == 0 ? C(0) : C(-lbm_w(q));
         } else {
-            // blocked directions of x (bit q: x + e_q outside the room or
-            // SOLID; 0 for an interior cell).  Slot q receives
-            //  (a) f*_q(x - e_q) when x - e_q = x + e_{-q} is not blocked;
-            //  (b) f*_OPP[q](x) when x's own direction OPP[q] is blocked.
-            // OPP of LBMSolver.cpp:27 pairs the diagonals as mirror images
-            // (7 <-> 8 is (1,1,0) <-> (-1,1,0)), so (a) and (b) are
-            // independent and a slot gets 0, 1 or 2 values.
-            const unsigned B = (fl & LF_REMAP) ? L.blk[o] : Bc;
-            // (a) for every slot, unconditionally: a blocked source reads the
-            // cell's own slot instead (a valid address) and is replaced below
+            const unsigned B = L.blk[o];
 #pragma unroll
             for (int q = 0; q < 19; q++) {
-                const int s = o - (c_ex(q) * plane + c_ey(q) * nz + c_ez(q));
-                fq[q] = C(S::ld(fa + (q * n + (((B >> c_rev(q)) & 1u) ? o : s))));
+                const int s = o - (c_ex(q) * plane + c_ey(q) * L.nz + c_ez(q));
+                fq[q] = C(S::ld(fa + ((size_t)q * L.np + (((B >> c_rev(q)) & 1u) ? o : s))));
             }
-            if (B) {
-                // cells next to a wall or SOLID: drop blocked sources, add (b)
+            if (B) fix_blocked<MODE>(L, fa, o, B, fq);
+        }
+        C vx, vy, vz;
+        double pc;
+        collide_cell<MODE>(L, c, L.ct[c], fq, vx, vy, vz, pc);
 #pragma unroll
-                for (int q = 0; q < 19; q++) {
-                    const int qq = c_opp(q);
-                    const bool ina = !((B >> c_rev(q)) & 1u);
-                    const bool inb = (B >> qq) & 1u;
-                    const C va = fq[q];
-                    const C vb = inb ? C(S::ld(fa + (qq * n + o))) : C(0);
-                    if (MODE == 0) {
-                        // the reference's zeroed slot plus what arrives
-                        fq[q] = ina ? (inb ? va + vb : va) : vb;
-                    } else {
-                        // shifted storage g = f - w (w_q == w_OPP[q]): two
-                        // arrivals give g_a + g_b + w, none gives -w
-                        fq[q] = ina ? (inb ? va + vb + C(lbm_w(q)) : va) : (inb ? vb : C(-lbm_w(q)));
-                    }
-                }
+        for (int q = 0; q < 19; q++) S::st(fb + ((size_t)q * L.np + c), fq[q]);
+        cu[c] = vx; cv[c] = vy; cw[c] = vz;
+        p[c] = pc;
+    }
+}
+
+// One fused step; see the file comment.  fa = f* of this step, fb = f* of
+// the next, cu/cv/cw = cell-centred velocity (m/s), p = rho*cs^2.
+//
+// NV cells c, c + 1 (c a multiple of NV) per thread.  Slot q of cell c comes
+// from f_q of cell c - e_q, at a distance that is the same for every cell, so
+// a pair of slots moves with one load where that distance is even and with
+// two where it is odd; PAR says which (0: the row length is even, 1: the row
+// length is odd and the plane even, 2: both odd).  A source outside the room
+// or SOLID is loaded like any other (the buffers have room before and after)
+// and replaced below.
+//
+// Bound: memory, 2 x 19 populations, four cell values and a flag per cell, as
+// long as enough loads are in flight.  One cell per thread in the narrow modes
+// issued 19 loads of 2 or 4 bytes each and was bound by instructions (FP32 641
+// us and FP16 591 at 384 x 320 x 128, now 497 and 394; 306 and 188 at 301 x 203
+// x 101, now 217 and 183): pairs halve the memory instructions and the packed
+// FP32 arithmetic halves the collision.  Where the row is odd most directions
+// keep two loads, so odd rows gain less.  Waiting for the type of the source
+// cell before its population cost the rest (the masks come first instead, and
+// only cells next to a wall look at one), as did one load after another of the
+// re-mapped cells inside a warp of ordinary ones.
+template <int MODE, int NV, int PAR>
+__global__ void __launch_bounds__(256, LbmLaunch<MODE, NV>::blocks)
+    k_lbm_step(LbmDev L, const typename Store<MODE>::T *f0, typename Store<MODE>::T *f1,
+               CellVel<MODE> *__restrict__ cu, CellVel<MODE> *__restrict__ cv, CellVel<MODE> *__restrict__ cw,
+               double *__restrict__ p, const LbmState *st, unsigned remap_blocks)
+{
+    using S = Store<MODE>;
+    using T = typename S::T;
+    using C = typename std::conditional<MODE == 0, double, float>::type;
+    if (st->halt) return;
+    const T *__restrict__ fa = st->par ? f1 : f0;
+    T *__restrict__ fb = st->par ? (T *)f0 : f1;
+    if (blockIdx.x < remap_blocks) {
+        step_remapped<MODE>(L, fa, fb, cu, cv, cw, p, blockIdx.x * blockDim.x + threadIdx.x, remap_blocks * blockDim.x);
+        return;
+    }
+    const int n = L.n, np = L.np, nz = L.nz, plane = L.ny * nz;
+    const unsigned items = (unsigned)(n + NV - 1) / NV, stride = (gridDim.x - remap_blocks) * blockDim.x;
+    // The flags of the next cells are loaded while these cells' populations
+    // are in flight, so each item waits for one round trip to memory only.
+    unsigned it = (blockIdx.x - remap_blocks) * blockDim.x + threadIdx.x;
+    auto flags = [&](unsigned i) -> unsigned {
+        if (NV == 1) return L.fl[i];
+        // (an odd lattice's last pair has one cell; the other counts as SOLID)
+        const unsigned c = 2 * i;
+        return c + 1 < (unsigned)n ? *reinterpret_cast<const uint16_t *>(L.fl + c) : L.fl[c] | ((unsigned)CT_SOLID << 8);
+    };
+    unsigned fl = it < items ? flags(it) : 0u, fln = 0;
+    for (; it < items; it += stride, fl = fln) {
+        if (it + stride < items) fln = flags(it + stride);
+        const unsigned c = it * NV;
+        // blocked directions of cells next to a wall (0 elsewhere)
+        unsigned B[NV];
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            const unsigned cf = (fl >> (8 * v)) & 0xffu;
+            B[v] = (cf & (LF_OPEN | LF_REMAP)) || (cf & 3u) == CT_SOLID ? 0u : L.blk[c + v];
+        }
+        C f[NV][19];
+#pragma unroll
+        for (int q = 0; q < 19; q++) {
+            const int off = c_ex(q) * plane + c_ey(q) * nz + c_ez(q);
+            // (pairs: 32-bit indices, or the 64-bit pointers of 38 streams take up the registers)
+            const T *src = NV == 1 ? fa + ((long long)q * np - off) + c : fa + (c + ((unsigned)(q * np) - (unsigned)off));
+            if constexpr (NV == 1) {
+                f[0][q] = C(S::ld(src));
+            } else if (constexpr_parity<PAR>(q)) {
+                f[0][q] = C(S::ld(src));
+                f[1][q] = C(S::ld(src + 1));
+            } else {
+                S::ld2(src, f[0][q], f[1][q]);
             }
         }
+        // cells next to a wall
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            if (B[v]) fix_blocked<MODE>(L, fa, (int)c + v, B[v], f[v]);
+        }
         // moments (LBMSolver.cpp:306-318) and next-step collision
-        if (MODE == 0) {
-            double rho = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
-#pragma unroll
-            for (int q = 0; q < 19; q++) add_moments<double>(q, fq[q], rho, ux, uy, uz);
-            if (rho > 1e-14) { ux /= rho; uy /= rho; uz /= rho; }
-            cu[c] = ux * L.l2p; cv[c] = uy * L.l2p; cw[c] = uz * L.l2p;
-            p[c] = rho * (1.0 / 3.0);
-            if (t == CT_INFLOW && L.fan_of[c] != 255) {
-                const double *fv = L.fan_lat + 3 * L.fan_of[c];
-#pragma unroll
-                for (int q = 0; q < 19; q++) S::st(fb + (q * n + c), feq64(q, 1.0, fv[0], fv[1], fv[2]));
-            } else if (t == CT_INFLOW) {
-#pragma unroll
-                for (int q = 0; q < 19; q++) S::st(fb + (q * n + c), fq[q]);
-            } else {
-                const double itau = 1.0 / L.tau;
-#pragma unroll
-                for (int q = 0; q < 19; q++) {
-                    const double fe = feq64(q, rho, ux, uy, uz);
-                    S::st(fb + (q * n + c), fq[q] + itau * (fe - fq[q]));
-                }
-            }
+        C vx[NV], vy[NV], vz[NV];
+        double pc[NV];
+        if constexpr (MODE != 0 && NV == 2) {
+            // (an INFLOW cell does not relax; a fan's equilibrium replaces it)
+            const bool in0 = (fl & 3u) == CT_INFLOW, in1 = ((fl >> 8) & 3u) == CT_INFLOW;
+            const float itau = (float)(1.0 / L.tau);
+            float u0[3], u1[3], d0, d1;
+            collide_pair(f[0], f[1], in0 ? 0.0f : itau, in1 ? 0.0f : itau, u0, u1, d0, d1);
+            vx[0] = (float)((double)u0[0] * L.l2p); vx[1] = (float)((double)u1[0] * L.l2p);
+            vy[0] = (float)((double)u0[1] * L.l2p); vy[1] = (float)((double)u1[1] * L.l2p);
+            vz[0] = (float)((double)u0[2] * L.l2p); vz[1] = (float)((double)u1[2] * L.l2p);
+            pc[0] = (double)(1.0f + d0) * (1.0 / 3.0);
+            pc[1] = (double)(1.0f + d1) * (1.0 / 3.0);
+            if (in0) inflow32(L, (int)c, f[0]);
+            if (in1) inflow32(L, (int)c + 1, f[1]);
         } else {
-            float drho = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
 #pragma unroll
-            for (int q = 0; q < 19; q++) add_moments<float>(q, fq[q], drho, jx, jy, jz);
-            const float rho = 1.0f + drho;
-            float ux = jx, uy = jy, uz = jz;
-            if (rho > 1e-14f) { ux /= rho; uy /= rho; uz /= rho; }
-            cu[c] = (float)((double)ux * L.l2p);
-            cv[c] = (float)((double)uy * L.l2p);
-            cw[c] = (float)((double)uz * L.l2p);
-            p[c] = (double)rho * (1.0 / 3.0);
-            if (t == CT_INFLOW && L.fan_of[c] != 255) {
-                const double *fv = L.fan_lat + 3 * L.fan_of[c];
+            for (int v = 0; v < NV; v++)
+                collide_cell<MODE>(L, (int)c + v, (fl >> (8 * v)) & 3u, f[v], vx[v], vy[v], vz[v], pc[v]);
+        }
 #pragma unroll
-                for (int q = 0; q < 19; q++)
-                    S::st(fb + (q * n + c), geq32(q, 0.0f, (float)fv[0], (float)fv[1], (float)fv[2]));
-            } else if (t == CT_INFLOW) {
+        for (int v = 0; v < NV; v++)
+            if (((fl >> (8 * v)) & 3u) == CT_SOLID) vx[v] = vy[v] = vz[v] = C(0);
+        // A SOLID cell's populations are never read, so they may be anything;
+        // its p stays as it is.  Nothing is stored for a re-mapped cell.
+        const bool w0 = !(fl & LF_REMAP), w1 = NV > 1 && !((fl >> 8) & LF_REMAP) && c + 1 < (unsigned)n;
+        const bool p0 = w0 && (fl & 3u) != CT_SOLID, p1 = w1 && ((fl >> 8) & 3u) != CT_SOLID;
+        if constexpr (NV == 1) {
+            if (w0) {
 #pragma unroll
-                for (int q = 0; q < 19; q++) S::st(fb + (q * n + c), fq[q]);
-            } else {
-                const float itau = (float)(1.0 / L.tau);
-#pragma unroll
-                for (int q = 0; q < 19; q++) {
-                    const float ge = geq32(q, drho, ux, uy, uz);
-                    S::st(fb + (q * n + c), fq[q] + itau * (ge - fq[q]));
-                }
+                for (int q = 0; q < 19; q++) S::st(fb + (size_t)q * np + c, f[0][q]);
+                cu[c] = vx[0]; cv[c] = vy[0]; cw[c] = vz[0];
+                if (p0) p[c] = pc[0];
             }
+        } else if (w0 && w1) {
+#pragma unroll
+            for (int q = 0; q < 19; q++) S::st2(fb + (c + (unsigned)(q * np)), f[0][q], f[1][q]);
+            Store<MODE == 0 ? 0 : 1>::st2(cu + c, vx[0], vx[1]);
+            Store<MODE == 0 ? 0 : 1>::st2(cv + c, vy[0], vy[1]);
+            Store<MODE == 0 ? 0 : 1>::st2(cw + c, vz[0], vz[1]);
+            if (p0 && p1) *reinterpret_cast<double2 *>(p + c) = make_double2(pc[0], pc[1]);
+            else if (p0) p[c] = pc[0];
+            else if (p1) p[c + 1] = pc[1];
+        } else if (w0 || w1) {
+            const unsigned o = w0 ? c : c + 1;
+#pragma unroll
+            for (int q = 0; q < 19; q++) S::st(fb + (o + (unsigned)(q * np)), w0 ? f[0][q] : f[1][q]);
+            cu[o] = w0 ? vx[0] : vx[1]; cv[o] = w0 ? vy[0] : vy[1]; cw[o] = w0 ? vz[0] : vz[1];
+            if (w0 ? p0 : p1) p[o] = w0 ? pc[0] : pc[1];
         }
     }
 }
@@ -323,7 +573,7 @@ __global__ void k_lbm_init(LbmDev L, typename Store<MODE>::T *f)
                 for (int q = 0; q < 19; q++) fq[q] += itau * (feq64(q, rho, ux, uy, uz) - fq[q]);
             }
 #pragma unroll
-            for (int q = 0; q < 19; q++) S::st(f + (size_t)q * n + c, fq[q]);
+            for (int q = 0; q < 19; q++) S::st(f + (size_t)q * L.np + c, fq[q]);
         } else {
             float g[19];
             const bool fan = t == CT_INFLOW && L.fan_of[c] != 255;
@@ -341,79 +591,21 @@ __global__ void k_lbm_init(LbmDev L, typename Store<MODE>::T *f)
                 for (int q = 0; q < 19; q++) g[q] += itau * (geq32(q, drho, jx / rho, jy / rho, jz / rho) - g[q]);
             }
 #pragma unroll
-            for (int q = 0; q < 19; q++) S::st(f + (size_t)q * n + c, g[q]);
+            for (int q = 0; q < 19; q++) S::st(f + (size_t)q * L.np + c, g[q]);
         }
     }
 }
 
-// Face velocities of extract_macroscopic (LBMSolver.cpp:333-375), max
-// |du| against the previous faces (LBMSolver.cpp:423-433) and max |div|
-// over FLUID cells (LBMSolver.cpp:382-396), cell-centric like k_correct.
-template <class V>
-__global__ void __launch_bounds__(256) k_lbm_faces(LbmDev L, const V *__restrict__ cu,
-                                                   const V *__restrict__ cv,
-                                                   const V *__restrict__ cw, double *__restrict__ u,
-                                                   double *__restrict__ v, double *__restrict__ w,
-                                                   LbmState *st)
+// StepResult and convergence test (LBMSolver.cpp:423-440), by one thread once
+// every block has folded its maxima in.
+__device__ __forceinline__ void lbm_finalize(double dt, double tol, LbmState *st, ffr_step_result *ring)
 {
-    __shared__ double sh[32];
-    if (st->halt) return;
-    const int nx = L.nx, ny = L.ny, nz = L.nz, plane = ny * nz;
-    double dmax = 0.0, divmax = 0.0;
-    for (Walk wk(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ny, nz, L.n); wk.ok(); wk.next()) {
-        const int c = wk.c, i = wk.i, j = wk.j, k = wk.k;
-        const int uf = c, vf = (i * (ny + 1) + j) * nz + k, wf = (i * ny + j) * (nz + 1) + k;
-        // every load first, then the arithmetic, then the stores
-        const double cuc = cu[c], cvc = cv[c], cwc = cw[c];
-        // neighbours through indices clamped into the arrays (the value is
-        // only used when the neighbour exists)
-        const int last = L.n - 1;
-        const double cum = cu[max(c - plane, 0)], cup = cu[min(c + plane, last)];
-        const double cvm = cv[max(c - nz, 0)], cvp = cv[min(c + nz, last)];
-        const double cwm = cw[max(c - 1, 0)], cwp = cw[min(c + 1, last)];
-        const double uo = u[uf], vo = v[vf], wo = w[wf];
-        const double uho = (i == nx - 1) ? u[uf + plane] : 0.0;
-        const double vho = (j == ny - 1) ? v[vf + nz] : 0.0;
-        const double who = (k == nz - 1) ? w[wf + 1] : 0.0;
-        const bool fluid = L.ct[c] == CT_FLUID;
-        const double ulo = (i == 0) ? cuc : 0.5 * (cum + cuc);
-        const double uhi = (i == nx - 1) ? cuc : 0.5 * (cuc + cup);
-        const double vlo = (j == 0) ? cvc : 0.5 * (cvm + cvc);
-        const double vhi = (j == ny - 1) ? cvc : 0.5 * (cvc + cvp);
-        const double wlo = (k == 0) ? cwc : 0.5 * (cwm + cwc);
-        const double whi = (k == nz - 1) ? cwc : 0.5 * (cwc + cwp);
-        dmax = fmax(dmax, fabs(ulo - uo));
-        dmax = fmax(dmax, fabs(vlo - vo));
-        dmax = fmax(dmax, fabs(wlo - wo));
-        if (i == nx - 1) dmax = fmax(dmax, fabs(uhi - uho));
-        if (j == ny - 1) dmax = fmax(dmax, fabs(vhi - vho));
-        if (k == nz - 1) dmax = fmax(dmax, fabs(whi - who));
-        if (fluid)
-            divmax = fmax(divmax, fabs((uhi - ulo) * L.idxv[i] + (vhi - vlo) * L.idyv[j] + (whi - wlo) * L.idzv[k]));
-        u[uf] = ulo;
-        v[vf] = vlo;
-        w[wf] = wlo;
-        if (i == nx - 1) u[uf + plane] = uhi;
-        if (j == ny - 1) v[vf + nz] = vhi;
-        if (k == nz - 1) w[wf + 1] = whi;
-    }
-    dmax = block_max(dmax, sh);
-    divmax = block_max(divmax, sh);
-    if (threadIdx.x == 0) {
-        atomic_max_nonneg(&st->dmax_bits, dmax);
-        atomic_max_nonneg(&st->div_bits, divmax);
-    }
-}
-
-__global__ void k_lbm_finalize(double dt, double tol, LbmState *st, ffr_step_result *ring)
-{
-    if (st->halt || threadIdx.x != 0) return;
-    const double vc = __longlong_as_double((long long)st->dmax_bits) / dt;
+    const double vc = __longlong_as_double((long long)__ldcg(&st->dmax_bits)) / dt;
     ffr_step_result r;
     r.step = st->step + 1;
     r.velocity_change = vc;
     r.pressure_residual = 0.0;
-    r.divergence_max = __longlong_as_double((long long)st->div_bits);
+    r.divergence_max = __longlong_as_double((long long)__ldcg(&st->div_bits));
     r.converged = vc < tol;
     r.T_mean = 0.0;
     r.cg_iterations = 0;
@@ -425,7 +617,136 @@ __global__ void k_lbm_finalize(double dt, double tol, LbmState *st, ffr_step_res
     st->dmax_bits = 0;
     st->div_bits = 0;
     st->flags = 0;
+    st->ticket = 0;
     if (r.converged && st->stop_on_converge) st->halt = 1;
+}
+
+// One value of each cell of a pair.
+__device__ __forceinline__ void load_cells(const double *p, double (&x)[2]) { Store<0>::ld2(p, x[0], x[1]); }
+__device__ __forceinline__ void load_cells(const float *p, float (&x)[2]) { Store<1>::ld2(p, x[0], x[1]); }
+
+// Face velocities of extract_macroscopic (LBMSolver.cpp:333-375), max
+// |du| against the previous faces (LBMSolver.cpp:423-433) and max |div|
+// over FLUID cells (LBMSolver.cpp:382-396), cell-centric like k_correct; the
+// last block closes the step.  PAIRS (even rows): the cells (k, k + 1) of a
+// pair at an even index, so the cell velocities and the x and y faces move
+// with one load or store per pair.  Every load comes first, then the
+// arithmetic, then the stores; neighbours through indices clamped into the
+// arrays (the value is only used when the neighbour exists).  Bound: memory
+// (the faces read and written, the cell velocities once), 4.6 TB/s of it in
+// pairs at 384 x 320 x 128.  Closing the step here takes a launch of 3 us off
+// every step (48.6 -> 47.1 us for a 25 x 20 x 12 one with its copies).
+template <class V, bool PAIRS>
+__global__ void __launch_bounds__(256) k_lbm_faces(LbmDev L, const V *__restrict__ cu,
+                                                   const V *__restrict__ cv,
+                                                   const V *__restrict__ cw, double *__restrict__ u,
+                                                   double *__restrict__ v, double *__restrict__ w,
+                                                   LbmState *st, double dt, double tol, ffr_step_result *ring)
+{
+    __shared__ double sh[32];
+    if (st->halt) return;
+    const int nx = L.nx, ny = L.ny, nz = L.nz, plane = ny * nz;
+    double dmax = 0.0, divmax = 0.0;
+    if constexpr (PAIRS) {
+        constexpr int NV = 2;
+        const int last = L.n - NV;
+        for (Walk wk(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ny, nz / NV, L.n / NV); wk.ok(); wk.next()) {
+            const int i = wk.i, j = wk.j, k = wk.k * NV, c = wk.c * NV;
+            const int uf = c, vf = (i * (ny + 1) + j) * nz + k, wf = (i * ny + j) * (nz + 1) + k;
+            V cuc[NV], cum[NV], cup[NV], cvc[NV], cvm[NV], cvp[NV], cwc[NV];
+            load_cells(cu + c, cuc);
+            load_cells(cu + max(c - plane, 0), cum);
+            load_cells(cu + min(c + plane, last), cup);
+            load_cells(cv + c, cvc);
+            load_cells(cv + max(c - nz, 0), cvm);
+            load_cells(cv + min(c + nz, last), cvp);
+            load_cells(cw + c, cwc);
+            const double cwm = cw[max(c - 1, 0)], cwp = cw[min(c + NV, L.n - 1)];
+            double uo[NV], vo[NV], wo[NV], uho[NV] = {}, vho[NV] = {};
+            load_cells(u + uf, uo);
+            load_cells(v + vf, vo);
+#pragma unroll
+            for (int a = 0; a < NV; a++) wo[a] = w[wf + a];
+            if (i == nx - 1) load_cells(u + uf + plane, uho);
+            if (j == ny - 1) load_cells(v + vf + nz, vho);
+            const double who = (k + NV == nz) ? w[wf + NV] : 0.0;
+            double ulo[NV], uhi[NV], vlo[NV], vhi[NV], wl[NV + 1];
+            wl[0] = (k == 0) ? (double)cwc[0] : 0.5 * (cwm + (double)cwc[0]);
+            wl[1] = 0.5 * ((double)cwc[0] + (double)cwc[NV - 1]);
+            wl[NV] = (k + NV == nz) ? (double)cwc[NV - 1] : 0.5 * ((double)cwc[NV - 1] + cwp);
+            if (k + NV == nz) dmax = fmax(dmax, fabs(wl[NV] - who));
+#pragma unroll
+            for (int a = 0; a < NV; a++) {
+                const double uc = cuc[a], vc = cvc[a];
+                ulo[a] = (i == 0) ? uc : 0.5 * ((double)cum[a] + uc);
+                uhi[a] = (i == nx - 1) ? uc : 0.5 * (uc + (double)cup[a]);
+                vlo[a] = (j == 0) ? vc : 0.5 * ((double)cvm[a] + vc);
+                vhi[a] = (j == ny - 1) ? vc : 0.5 * (vc + (double)cvp[a]);
+                dmax = fmax(dmax, fabs(ulo[a] - uo[a]));
+                dmax = fmax(dmax, fabs(vlo[a] - vo[a]));
+                dmax = fmax(dmax, fabs(wl[a] - wo[a]));
+                if (i == nx - 1) dmax = fmax(dmax, fabs(uhi[a] - uho[a]));
+                if (j == ny - 1) dmax = fmax(dmax, fabs(vhi[a] - vho[a]));
+                if (L.ct[c + a] == CT_FLUID)
+                    divmax = fmax(divmax, fabs((uhi[a] - ulo[a]) * L.idxv[i] + (vhi[a] - vlo[a]) * L.idyv[j] +
+                                               (wl[a + 1] - wl[a]) * L.idzv[k + a]));
+            }
+            Store<0>::st2(u + uf, ulo[0], ulo[1]);
+            Store<0>::st2(v + vf, vlo[0], vlo[1]);
+#pragma unroll
+            for (int a = 0; a < NV; a++) w[wf + a] = wl[a];
+            if (i == nx - 1) Store<0>::st2(u + uf + plane, uhi[0], uhi[1]);
+            if (j == ny - 1) Store<0>::st2(v + vf + nz, vhi[0], vhi[1]);
+            if (k + NV == nz) w[wf + NV] = wl[NV];
+        }
+    } else {
+        for (Walk wk(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ny, nz, L.n); wk.ok(); wk.next()) {
+            const int c = wk.c, i = wk.i, j = wk.j, k = wk.k;
+            const int uf = c, vf = (i * (ny + 1) + j) * nz + k, wf = (i * ny + j) * (nz + 1) + k;
+            // every load first, then the arithmetic, then the stores
+            const double cuc = cu[c], cvc = cv[c], cwc = cw[c];
+            // neighbours through indices clamped into the arrays (the value is
+            // only used when the neighbour exists)
+            const int last = L.n - 1;
+            const double cum = cu[max(c - plane, 0)], cup = cu[min(c + plane, last)];
+            const double cvm = cv[max(c - nz, 0)], cvp = cv[min(c + nz, last)];
+            const double cwm = cw[max(c - 1, 0)], cwp = cw[min(c + 1, last)];
+            const double uo = u[uf], vo = v[vf], wo = w[wf];
+            const double uho = (i == nx - 1) ? u[uf + plane] : 0.0;
+            const double vho = (j == ny - 1) ? v[vf + nz] : 0.0;
+            const double who = (k == nz - 1) ? w[wf + 1] : 0.0;
+            const bool fluid = L.ct[c] == CT_FLUID;
+            const double ulo = (i == 0) ? cuc : 0.5 * (cum + cuc);
+            const double uhi = (i == nx - 1) ? cuc : 0.5 * (cuc + cup);
+            const double vlo = (j == 0) ? cvc : 0.5 * (cvm + cvc);
+            const double vhi = (j == ny - 1) ? cvc : 0.5 * (cvc + cvp);
+            const double wlo = (k == 0) ? cwc : 0.5 * (cwm + cwc);
+            const double whi = (k == nz - 1) ? cwc : 0.5 * (cwc + cwp);
+            dmax = fmax(dmax, fabs(ulo - uo));
+            dmax = fmax(dmax, fabs(vlo - vo));
+            dmax = fmax(dmax, fabs(wlo - wo));
+            if (i == nx - 1) dmax = fmax(dmax, fabs(uhi - uho));
+            if (j == ny - 1) dmax = fmax(dmax, fabs(vhi - vho));
+            if (k == nz - 1) dmax = fmax(dmax, fabs(whi - who));
+            if (fluid)
+                divmax = fmax(divmax, fabs((uhi - ulo) * L.idxv[i] + (vhi - vlo) * L.idyv[j] + (whi - wlo) * L.idzv[k]));
+            u[uf] = ulo;
+            v[vf] = vlo;
+            w[wf] = wlo;
+            if (i == nx - 1) u[uf + plane] = uhi;
+            if (j == ny - 1) v[vf + nz] = vhi;
+            if (k == nz - 1) w[wf + 1] = whi;
+        }
+    }
+    dmax = block_max(dmax, sh);
+    divmax = block_max(divmax, sh);
+    if (threadIdx.x == 0) {
+        atomic_max_nonneg(&st->dmax_bits, dmax);
+        atomic_max_nonneg(&st->div_bits, divmax);
+        // the block that arrives last closes the step
+        __threadfence();
+        if (atomicAdd(&st->ticket, 1u) == gridDim.x - 1) lbm_finalize(dt, tol, st, ring);
+    }
 }
 
 __global__ void k_lbm_divergence(LbmDev L, const double *u, const double *v, const double *w,
@@ -505,7 +826,7 @@ __global__ void k_lbm_fan_of(const uint8_t *__restrict__ ct, int nx, int ny, int
 // exported as 0, the value the reference's push streaming leaves in them
 // (LBMSolver.cpp:151-190), and never read by a step.
 template <int MODE>
-__global__ void k_lbm_export(int n, const uint8_t *__restrict__ ct, const typename Store<MODE>::T *__restrict__ f,
+__global__ void k_lbm_export(int n, int np, const uint8_t *__restrict__ ct, const typename Store<MODE>::T *__restrict__ f,
                              double *__restrict__ out)
 {
     const long long total = 19ll * n;
@@ -515,7 +836,7 @@ __global__ void k_lbm_export(int n, const uint8_t *__restrict__ ct, const typena
         const int c = (int)(t - (long long)q * n);
         double v = 0.0;
         if (ct[c] != CT_SOLID) {
-            v = (double)Store<MODE>::ld(f + t);
+            v = (double)Store<MODE>::ld(f + ((size_t)q * np + c));
             if (MODE != 0) v += lbm_w(q);
         }
         out[t] = v;
@@ -523,16 +844,17 @@ __global__ void k_lbm_export(int n, const uint8_t *__restrict__ ct, const typena
 }
 
 template <int MODE>
-__global__ void k_lbm_import(int n, const double *__restrict__ in, typename Store<MODE>::T *__restrict__ f)
+__global__ void k_lbm_import(int n, int np, const double *__restrict__ in, typename Store<MODE>::T *__restrict__ f)
 {
     const long long total = 19ll * n;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         const int q = (int)(t / n);
+        const size_t at = (size_t)q * np + (size_t)(t - (long long)q * n);
         const double v = in[t];
-        if (MODE == 0) Store<0>::st(reinterpret_cast<double *>(f) + t, v);
-        else if (MODE == 1) reinterpret_cast<float *>(f)[t] = (float)(v - lbm_w(q));
-        else reinterpret_cast<__half *>(f)[t] = __double2half(v - lbm_w(q));
+        if (MODE == 0) Store<0>::st(reinterpret_cast<double *>(f) + at, v);
+        else if (MODE == 1) reinterpret_cast<float *>(f)[at] = (float)(v - lbm_w(q));
+        else reinterpret_cast<__half *>(f)[at] = __double2half(v - lbm_w(q));
     }
 }
 
@@ -576,38 +898,51 @@ struct ffr_lbm {
 
 namespace {
 
+template <int MODE, int NV> void launch_step(ffr_lbm *s)
+{
+    using T = typename Store<MODE>::T;
+    using V = CellVel<MODE>;
+    const int par = (s->L.nz & 1) == 0 ? 0 : ((s->L.ny & 1) == 0 ? 1 : 2);
+    auto *fn = par == 0 || NV == 1 ? k_lbm_step<MODE, NV, 0> : (par == 1 ? k_lbm_step<MODE, NV, 1> : k_lbm_step<MODE, NV, 2>);
+    const unsigned blocks = blocks_for((s->L.n + NV - 1) / NV);
+    // the re-mapped cells have the first blocks to themselves
+    const unsigned rb = (unsigned)((s->L.nremap + kThr - 1) / kThr);
+    fn<<<blocks + rb, kThr, 0, s->stream>>>(s->L, (const T *)s->f0, (T *)s->f1, (V *)s->cu, (V *)s->cv, (V *)s->cw, s->p, s->st,
+                                          rb);
+}
+
+template <class V> void launch_faces(ffr_lbm *s)
+{
+    // pairs where the lattice is large enough to fill the GPU with them (15.7 M
+    // cells, FP32: 237 us singly, 214 in pairs; 4.8 M: 78 both; 1.7 M: 34 and 37)
+    const bool pairs = (s->L.nz & 1) == 0 && s->L.n >= 6000000;
+    auto *fn = pairs ? k_lbm_faces<V, true> : k_lbm_faces<V, false>;
+    fn<<<blocks_for(s->L.n / (pairs ? 2 : 1)), kThr, 0, s->stream>>>(s->L, (const V *)s->cu, (const V *)s->cv, (const V *)s->cw,
+                                                                    s->u, s->v, s->w, s->st, s->dt, s->tol, s->ring);
+}
+
 int lbm_enqueue(ffr_lbm *s)
 {
     cudaStream_t st = s->stream;
     s->prof.begin(FFR_LPROF_STREAM_COLLIDE, st);
     switch (s->storage) {
+    // FP64 pairs need 126 registers: fewer warps, which a small lattice misses
+    // (820 k cells: 59 us singly, 63 in pairs; 1.7 M: 109 both; 4.8 M: 321 and
+    // 313; 15.7 M: 1131 and 944)
     case FFR_LBM_FP64:
-        k_lbm_step<0><<<s->blocks, kThr, 0, st>>>(s->L, (const double *)s->f0, (double *)s->f1,
-                                                    (CellVel<0> *)s->cu, (CellVel<0> *)s->cv,
-                                                    (CellVel<0> *)s->cw, s->p, s->st);
+        if (s->L.n < 1500000) launch_step<0, 1>(s);
+        else launch_step<0, 2>(s);
         break;
-    case FFR_LBM_FP32:
-        k_lbm_step<1><<<s->blocks, kThr, 0, st>>>(s->L, (const float *)s->f0, (float *)s->f1,
-                                                    (CellVel<1> *)s->cu, (CellVel<1> *)s->cv,
-                                                    (CellVel<1> *)s->cw, s->p, s->st);
-        break;
-    default:
-        k_lbm_step<2><<<s->blocks, kThr, 0, st>>>(s->L, (const __half *)s->f0, (__half *)s->f1,
-                                                    (CellVel<2> *)s->cu, (CellVel<2> *)s->cv,
-                                                    (CellVel<2> *)s->cw, s->p, s->st);
+    case FFR_LBM_FP32: launch_step<1, 2>(s); break;
+    default: launch_step<2, 2>(s);
     }
     FFR_LAUNCHED(1);
     s->prof.end(st, 1);
     s->prof.begin(FFR_LPROF_FACES, st);
-    if (s->storage == FFR_LBM_FP64)
-        k_lbm_faces<double><<<s->blocks, kThr, 0, st>>>(s->L, s->cu, s->cv, s->cw, s->u, s->v, s->w, s->st);
-    else
-        k_lbm_faces<float><<<s->blocks, kThr, 0, st>>>(s->L, (const float *)s->cu, (const float *)s->cv,
-                                                       (const float *)s->cw, s->u, s->v, s->w, s->st);
+    if (s->storage == FFR_LBM_FP64) launch_faces<double>(s);
+    else launch_faces<float>(s);
     FFR_LAUNCHED(1);
-    k_lbm_finalize<<<1, 32, 0, st>>>(s->dt, s->tol, s->st, s->ring);
-    FFR_LAUNCHED(1);
-    s->prof.end(st, 2);
+    s->prof.end(st, 1);
     return FFR_OK;
 }
 
@@ -674,6 +1009,10 @@ int ffr_lbm_create(const ffr_room_desc *room, double tau, int max_steps, double 
     int rc = load_room(room, s->room);
     if (rc) { delete s; return rc; }
     const RoomGeom &g = s->room.g;
+    // a direction's populations: an even number (pairs stay aligned); the
+    // buffers continue by one plane, one row and a pair past the last
+    // direction, which the unconditional loads of boundary cells reach
+    const long long np = (g.n + 31) & ~31ll, ftotal = 19 * np + (long long)g.ny * g.nz + g.nz + 64;
     if (19ll * g.n >= (1ll << 31)) { delete s; return fail(FFR_ERANGE, "lattice too large (19*N >= 2^31)"); }
     s->storage = storage; s->tau = tau; s->dt = dt; s->tol = convergence_tol; s->max_steps = max_steps;
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -689,15 +1028,15 @@ int ffr_lbm_create(const ffr_room_desc *room, double tau, int max_steps, double 
     resolve_remap(s->room, rd, rs);
     const size_t es = storage == FFR_LBM_FP64 ? 8 : (storage == FFR_LBM_FP32 ? 4 : 2);
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t bytes = 2 * al(es * 19 * g.n) + 4 * al(8 * g.n) + al(8 * g.nu) + al(8 * g.nv) +
+    const size_t bytes = 2 * al(es * ftotal) + 4 * al(8 * g.n) + al(8 * g.nu) + al(8 * g.nv) +
                          al(8 * g.nw) + 3 * al(g.n) + al(4 * g.n) + al(8 * fan_lat.size()) + 2 * al(4 * (rd.size() + 1)) +
                          2 * (al(8 * g.nx) + al(8 * g.ny) + al(8 * g.nz)) + al(sizeof(LbmState)) +
                          al(sizeof(ffr_step_result) * kRingL) + al(8);
     rc = s->arena.alloc(bytes, s->stream);
     if (rc) { cudaStreamDestroy(s->stream); delete s; return rc; }
     Arena &a = s->arena;
-    s->f0 = a.take<char>(es * 19 * g.n);
-    s->f1 = a.take<char>(es * 19 * g.n);
+    s->f0 = a.take<char>(es * ftotal);
+    s->f1 = a.take<char>(es * ftotal);
     s->cu = a.take<double>(g.n); s->cv = a.take<double>(g.n); s->cw = a.take<double>(g.n);
     s->p = a.take<double>(g.n);
     s->u = a.take<double>(g.nu); s->v = a.take<double>(g.nv); s->w = a.take<double>(g.nw);
@@ -763,7 +1102,7 @@ int ffr_lbm_create(const ffr_room_desc *room, double tau, int max_steps, double 
         return rc;
     }
     FFR_CUDA(cudaMemsetAsync(s->st, 0, sizeof(LbmState), st));
-    s->L = LbmDev{nx, ny, nz, (int)g.n, (int)g.nu, (int)g.nv, (int)g.nw, ct, fld, blk, fo, fl, rdd, rsd,
+    s->L = LbmDev{nx, ny, nz, (int)g.n, (int)g.nu, (int)g.nv, (int)g.nw, (int)np, ct, fld, blk, fo, fl, rdd, rsd,
                   (int)rd.size(), dxv, dyv, dzv, idxv, idyv, idzv, tau, (g.lx / g.nx) / dt};
     s->blocks = blocks_for(g.n);
     switch (storage) {
@@ -903,9 +1242,9 @@ static int lbm_state_io(ffr_lbm *s, double *host_out, const double *host_in, int
     const int n = (int)s->room.g.n;
     if (host_out) {
         switch (s->storage) {
-        case FFR_LBM_FP64: k_lbm_export<0><<<nb, kThr, 0, s->stream>>>(n, s->L.ct, (const double *)cur, tmp); break;
-        case FFR_LBM_FP32: k_lbm_export<1><<<nb, kThr, 0, s->stream>>>(n, s->L.ct, (const float *)cur, tmp); break;
-        default: k_lbm_export<2><<<nb, kThr, 0, s->stream>>>(n, s->L.ct, (const __half *)cur, tmp);
+        case FFR_LBM_FP64: k_lbm_export<0><<<nb, kThr, 0, s->stream>>>(n, s->L.np, s->L.ct, (const double *)cur, tmp); break;
+        case FFR_LBM_FP32: k_lbm_export<1><<<nb, kThr, 0, s->stream>>>(n, s->L.np, s->L.ct, (const float *)cur, tmp); break;
+        default: k_lbm_export<2><<<nb, kThr, 0, s->stream>>>(n, s->L.np, s->L.ct, (const __half *)cur, tmp);
         }
         FFR_LAUNCHED(1);
         rc = staged_copy(host_out, tmp, 8 * total, true, s->stream);
@@ -914,9 +1253,9 @@ static int lbm_state_io(ffr_lbm *s, double *host_out, const double *host_in, int
         rc = staged_copy(tmp, host_in, 8 * total, false, s->stream);
         if (!rc) {
             switch (s->storage) {
-            case FFR_LBM_FP64: k_lbm_import<0><<<nb, kThr, 0, s->stream>>>(n, tmp, (double *)cur); break;
-            case FFR_LBM_FP32: k_lbm_import<1><<<nb, kThr, 0, s->stream>>>(n, tmp, (float *)cur); break;
-            default: k_lbm_import<2><<<nb, kThr, 0, s->stream>>>(n, tmp, (__half *)cur);
+            case FFR_LBM_FP64: k_lbm_import<0><<<nb, kThr, 0, s->stream>>>(n, s->L.np, tmp, (double *)cur); break;
+            case FFR_LBM_FP32: k_lbm_import<1><<<nb, kThr, 0, s->stream>>>(n, s->L.np, tmp, (float *)cur); break;
+            default: k_lbm_import<2><<<nb, kThr, 0, s->stream>>>(n, s->L.np, tmp, (__half *)cur);
             }
             FFR_LAUNCHED(1);
             if (step_io) {
