@@ -146,10 +146,10 @@ __device__ __forceinline__ void oc_neighbours(const OcLevel &L, int m, int c, un
 
 __device__ __forceinline__ float oc_sum(const float (&t)[6], const float (&v)[6])
 {
+    // (the choice is made on v: it stays off the chain of sums)
     float s = 0.0f;
 #pragma unroll
-    for (int a = 0; a < 6; a++)
-        if (t[a] != 0.0f) s += t[a] * v[a];
+    for (int a = 0; a < 6; a++) s += t[a] * (t[a] != 0.0f ? v[a] : 0.0f);
     return s;
 }
 
@@ -182,11 +182,30 @@ __device__ __forceinline__ void oc_set(const OcLevel &L, int m, int c, float val
     }
 }
 
+// The threads that work on a level: the cluster's, or the first n of block 0
+// (as many warps as the level has pairs for; those of the next coarser level are
+// among them).  A barrier of each level, of its own number, holds them together;
+// a thread that the next level does not need goes on to wait there.
+struct OcTeam {
+    int id, n;      // id < 0: the cluster
+    __device__ __forceinline__ void sync() const
+    {
+        // (shared memory only crosses blocks, so no device-wide fence)
+        if (id < 0) cooperative_groups::this_cluster().sync();
+        else if (n == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+    }
+};
+
 // One half sweep over the cells of colour c, by threads t of nt; `share`: the
 // boundary planes to the neighbours.
 template <bool FINE>
-__device__ __noinline__ void oc_sweep(const MGDev &M, const OcLevel &L, int c, int t, int nt, int rank, bool share)
+__device__ __noinline__ void oc_sweep(const MGDev &M, const OcLevel &L_, int c, int t, int nt, int rank, bool share)
 {
+    // (in registers: every field fetched again for a pair is a round trip to
+    // shared memory; a half sweep of 1600 pairs per block went from 4.6 k to 3.4 k
+    // cycles without them)
+    const OcLevel L = L_;
     for (int m = t; m < L.n; m += nt) {
         const unsigned f = L.flags()[m];
         float tt[6], v[6];
@@ -200,8 +219,9 @@ __device__ __noinline__ void oc_sweep(const MGDev &M, const OcLevel &L, int c, i
 // Residuals of the red cells (0 where there is no unknown), pair by pair, to
 // res of block `to` (this block's own: to == rank).
 template <bool FINE>
-__device__ __noinline__ void oc_residual(const MGDev &M, const OcLevel &L, float *res, int t, int nt, int rank, int to)
+__device__ __noinline__ void oc_residual(const MGDev &M, const OcLevel &L_, float *res, int t, int nt, int rank, int to)
 {
+    const OcLevel L = L_;
     for (int m = t; m < L.n; m += nt) {
         const unsigned f = L.flags()[m];
         float tt[6], v[6];
@@ -214,32 +234,92 @@ __device__ __noinline__ void oc_residual(const MGDev &M, const OcLevel &L, float
     }
 }
 
+// What a level's smoothing does besides its sweeps.
+enum : unsigned { OS_UP = 1,       // after the prolongation (else before the restriction)
+                  OS_SHARE = 2,    // boundary planes go to the neighbours
+                  OS_TOP = 4 };    // the first level on chip: its last sweep needs no halo
+
+// All half sweeps of one visit of a level of at most one pair per thread (not
+// level 0), and on the way down the red residuals (as oc_residual): the pair's
+// rows, right-hand sides and place are loaded once and stay in registers, which
+// took a half sweep of the lone block from 0.9 k cycles to 0.3 k.  Not for more
+// pairs per thread: three in registers measured 10 % slower per iteration than
+// oc_sweep (the code grows with them, and every pass of a V-cycle runs once, so
+// it is the fetching of instructions that then bounds it).
+__device__ __noinline__ void oc_smooth(const MGDev &M, const OcLevel &L_, unsigned what, OcTeam team, int t, int rank,
+                                       float *res, int to)
+{
+    const OcLevel L = L_;
+    const int n = L.n, rp = L.rp, pk = L.pk, m = max(0, min(t, n - 1));
+    float *const x0 = L.x(0) + rp + m, *const x1 = L.x(1) + rp + m;
+    const unsigned f = t < n ? L.flags()[m] : 0u;
+    const float b[2] = {L.b(0)[m], L.b(1)[m]}, D[2] = {L.D(0)[m], L.D(1)[m]};
+    float row[2][6];
+    oc_row<false>(M, L, m, 0, f, row[0]);
+    oc_row<false>(M, L, m, 1, f, row[1]);
+    const int h = (int)(f & 1u);
+    auto sum = [&](int c) {
+        const float *o = c ? x0 : x1;
+        const int z = h ^ c;
+        const float v[6] = {o[-rp], o[rp], o[-pk], o[pk], o[z - 1], o[z]};
+        return oc_sum(row[c], v);
+    };
+    auto half = [&](int c, bool share) {
+        const float val = (b[c] + sum(c)) / D[c];
+        if (f & (OF_RED << c)) oc_set(L, m, c, val, rank, share && (what & OS_SHARE));
+    };
+    const bool up = what & OS_UP;
+    for (int s = 0; s < kSmoothSweeps; s++) {
+        const bool end = s + 1 == kSmoothSweeps, last = up && end && (what & OS_TOP);
+        half(1, true);
+        team.sync();
+        if (!up && end) break;
+        half(0, !last);
+        if (!(last && (what & OS_SHARE))) team.sync();
+    }
+    if (up || t >= n) return;
+    const float r = f & OF_RED ? b[0] - (D[0] * *x0 - sum(0)) : 0.0f;
+    if (to == rank) res[m] = r;
+    else oc_store_peer(res + m, to, r);
+}
+
 // Right-hand side and first red sweep of level C from the residuals of the
 // finer level L's red cells (res: planes i0 on), summed in the order of a
 // nested loop over the children.
 __device__ __noinline__ void oc_coarse_rhs(const OcLevel &L, int i0, const float *res, const OcLevel &C, int t, int nt,
                                            int rank, bool share)
 {
-    for (int m = t; m < C.n; m += nt) {
+    // (in registers: every field of L that a test below had to fetch again was
+    // a round trip to shared memory, 4.8 k cycles for a level of one pair per thread)
+    const int nx = L.nx, ny = L.ny, nz = L.nz, sx = L.sx, sy = L.sy, sz = L.sz, pk = L.pk, rp = L.rp;
+    const int cnz = C.nz, n = C.n;
+    float *const cb[2] = {C.b(0), C.b(1)}, *const cD[2] = {C.D(0), C.D(1)};
+    for (int m = t; m < n; m += nt) {
         const OcItem it(C, m);
+        const int i = it.i << sx, j = it.j << sy, par = (it.i + it.j) & 1;
+        float r[2][8];
+#pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int K = 2 * it.p + h, c = ((it.i + it.j) & 1) ^ h;
-            if (K >= C.nz) continue;
-            float r[8];
+            const int k = (2 * it.p + h) << sz;
+            const int at = (i - i0) * rp + j * pk + (k >> 1), up = k & 1;
 #pragma unroll
             for (int q = 0; q < 8; q++) {
                 // the red children inside the level
                 const int a = q >> 2, b = (q >> 1) & 1, e = q & 1;
-                const int i = (it.i << L.sx) + a, j = (it.j << L.sy) + b, k = (K << L.sz) + e;
-                const bool use = a <= L.sx && b <= L.sy && e <= L.sz && i < L.nx && j < L.ny && k < L.nz &&
-                                 ((i + j + k) & 1) == 0;
-                r[q] = use ? res[(i - i0) * L.rp + j * L.pk + (k >> 1)] : 0.0f;
+                const bool use = (a <= sx) & (b <= sy) & (e <= sz) & (i + a < nx) & (j + b < ny) & (k + e < nz) &
+                                 (((i + j + k + a + b + e) & 1) == 0);
+                r[h][q] = use ? res[at + a * rp + b * pk + ((up + e) >> 1)] : 0.0f;
             }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int c = par ^ h;
+            if (2 * it.p + h >= cnz) continue;
             float sum = 0.0f;
 #pragma unroll
-            for (int q = 0; q < 8; q++) sum += r[q];
-            const float DP = C.D(c)[m];
-            C.b(c)[m] = sum;
+            for (int q = 0; q < 8; q++) sum += r[h][q];
+            const float DP = cD[c][m];
+            cb[c][m] = sum;
             oc_set(C, m, c, c == 0 && DP != 0.0f ? sum / DP : 0.0f, rank, share);
         }
     }
@@ -251,16 +331,17 @@ __device__ __noinline__ void oc_coarse_rhs(const OcLevel &L, int i0, const float
 // at `copy`, from plane `first` on.
 __device__ __noinline__ void oc_prolong(const OcLevel &L, const OcLevel &C, int copy, int first, int count, int t, int nt)
 {
-    float *x = L.x(0);
-    const unsigned char *flags = L.flags();
+    float *const x = L.x(0);
+    const unsigned char *const flags = L.flags();
     const int base = copy < 0 ? C.base + (1 - C.p0) * C.rp : copy - first * C.rp, stride = copy < 0 ? C.h2 : count;
-    for (int e = t; e < L.n + 2 * L.rp && L.n > 0; e += nt) {
+    const int n = L.n, rp = L.rp, nx = L.nx, nz = L.nz, sx = L.sx, sy = L.sy, sz = L.sz, crp = C.rp, cpk = C.pk;
+    for (int e = t; e < n + 2 * rp && n > 0; e += nt) {
         const OcItem it(L, e, -1);
-        const int k = 2 * it.p + ((it.i + it.j) & 1), m = e - L.rp;
-        if (it.i < 0 || it.i >= L.nx || k >= L.nz) continue;
-        if (m >= 0 && m < L.n && !(flags[m] & OF_RED)) continue;
-        const int I = it.i >> L.sx, J = it.j >> L.sy, K = k >> L.sz;
-        x[e] += oc_smem[base + ((I + J + K) & 1) * stride + I * C.rp + J * C.pk + (K >> 1)];
+        const int k = 2 * it.p + ((it.i + it.j) & 1), m = e - rp;
+        if ((it.i < 0) | (it.i >= nx) | (k >= nz)) continue;
+        if (m >= 0 && m < n && !(flags[m] & OF_RED)) continue;
+        const int I = it.i >> sx, J = it.j >> sy, K = k >> sz;
+        x[e] += oc_smem[base + ((I + J + K) & 1) * stride + I * crp + J * cpk + (K >> 1)];
     }
 }
 
@@ -305,50 +386,55 @@ __device__ __noinline__ void oc_setup(const PCGArgs &A, const OnchipPlan &Q, int
     if (t >= Q.lo && t < M.nlev) S.lv[t] = oc_level(M, Q, t, rank);
     __syncthreads();
     for (int l = Q.lo; l < M.nlev; l++) {
-        const OcLevel &L = S.lv[l];
+        const OcLevel L = S.lv[l];
         if (L.n == 0) continue;
         // one plane below the own ones as well
-        const int first = (l == 0 || L.p0 == 0) ? 0 : -1;
-        for (int e = t; e < L.n - first * L.rp; e += nt) {
-            const OcItem it(L, e, first);
-            const int m = e + first * L.rp;
-            const int par = (it.i + it.j) & 1;
-            unsigned f = (par ? OF_PAR : 0u) | (it.p == 0 ? OF_FIRST : 0u);
+        const int first = (l == 0 || L.p0 == 0) ? 0 : -1, count = L.n - first * L.rp;
+        const float4 *const coef = M.lv[l].coef;
+        constexpr int U = 4;      // pairs in flight
+        for (int e0 = t; e0 < count; e0 += U * nt) {
+            float4 cf[U][2];
+            unsigned code[U][2];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int k = 2 * it.p + h, c = par ^ h;      // colour of cell k
-                if (k >= L.nz) continue;
-                const int cell = (it.i * L.ny + it.j) * L.nz + k;
-                if (l == 0) {
-                    const unsigned code = A.R.sc[cell];
-                    float tt[6], D;
-                    fine_coefs(M, code, it.i, it.j, k, tt, D);
-                    L.code(c)[m] = (unsigned short)code;
-                    L.D(c)[m] = D;
-                    if (active_code(code)) f |= OF_RED << c;
-                } else {
-                    const float4 cf = M.lv[l].coef[cell];
-                    if (cf.w != 0.0f) f |= OF_RED << c;
-                    L.t(0, c)[L.rp + m] = cf.x;
-                    L.t(1, c)[L.rp + m] = cf.y;
-                    L.t(2, c)[L.rp + m] = cf.z;
-                    if (m >= 0) L.D(c)[m] = cf.w;
+            for (int u = 0; u < U; u++) {
+                const OcItem it(L, min(e0 + u * nt, count - 1), first);
+                const int cell = (it.i * L.ny + it.j) * L.nz + 2 * it.p, two = 2 * it.p + 1 < L.nz;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    if (l == 0) code[u][h] = A.R.sc[cell + h * two];
+                    else cf[u][h] = coef[cell + h * two];
                 }
             }
-            if (m >= 0) L.flags()[m] = (unsigned char)f;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int e = e0 + u * nt, m = e + first * L.rp;
+                if (e >= count) break;
+                const OcItem it(L, e, first);
+                const int par = (it.i + it.j) & 1;
+                unsigned f = (par ? OF_PAR : 0u) | (it.p == 0 ? OF_FIRST : 0u);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int k = 2 * it.p + h, c = par ^ h;      // colour of cell k
+                    if (k >= L.nz) continue;
+                    if (l == 0) {
+                        float tt[6], D;
+                        fine_coefs(M, code[u][h], it.i, it.j, k, tt, D);
+                        L.code(c)[m] = (unsigned short)code[u][h];
+                        L.D(c)[m] = D;
+                        if (active_code(code[u][h])) f |= OF_RED << c;
+                    } else {
+                        if (cf[u][h].w != 0.0f) f |= OF_RED << c;
+                        L.t(0, c)[L.rp + m] = cf[u][h].x;
+                        L.t(1, c)[L.rp + m] = cf[u][h].y;
+                        L.t(2, c)[L.rp + m] = cf[u][h].z;
+                        if (m >= 0) L.D(c)[m] = cf[u][h].w;
+                    }
+                }
+                if (m >= 0) L.flags()[m] = (unsigned char)f;
+            }
         }
     }
     __syncthreads();
-}
-
-// Barriers: of the cluster (shared memory only crosses blocks, so no
-// device-wide fence), of the block, of one warp.
-enum OcGroup { OC_CLUSTER, OC_BLOCK, OC_WARP };
-__device__ __forceinline__ void oc_sync(OcGroup g)
-{
-    if (g == OC_CLUSTER) cooperative_groups::this_cluster().sync();
-    else if (g == OC_BLOCK) __syncthreads();
-    else __syncwarp();
 }
 
 // The V-cycle of levels lo .. nlev-1: level lo's right-hand side and first red
@@ -361,7 +447,7 @@ __device__ __noinline__ void oc_vcycle(const PCGArgs &A, const OnchipPlan &Q, in
 {
     const MGDev &M = A.M;
     const int t = threadIdx.x, nt = blockDim.x, last = M.nlev - 1;
-    const OcGroup all = Q.blocks == 1 || Q.fb == Q.lo ? OC_BLOCK : OC_CLUSTER;
+    const bool lone = Q.blocks == 1 || Q.fb == Q.lo;
     float *red = oc_smem + Q.off_red, *res0 = oc_smem + Q.off_res;
     auto sweep = [&](int l, int c, int n, bool share) {
         if (FINE && l == 0) oc_sweep<true>(M, S.lv[l], c, t, n, rank, share);
@@ -371,79 +457,107 @@ __device__ __noinline__ void oc_vcycle(const PCGArgs &A, const OnchipPlan &Q, in
         if (FINE && l == 0) oc_residual<true>(M, S.lv[l], res, t, n, rank, to);
         else oc_residual<false>(M, S.lv[l], res, t, n, rank, to);
     };
+    const OcTeam all{lone ? 0 : -1, nt};
+    auto team_of = [&](int l) {
+        return l < Q.fb ? all : OcTeam{1 + l - Q.fb, min(nt, (S.lv[l].nx * S.lv[l].rp + 31) & ~31)};
+    };
+    // one visit of a level: its half sweeps, on the way down the residuals too
+    auto smooth = [&](int l, const OcTeam &T, bool up, float *res, int to) {
+        const OcLevel &L = S.lv[l];
+        const bool split = l < Q.fb, top = l == Q.lo;
+        if (l > 0 && L.own <= T.n) {
+            const unsigned what = (up ? OS_UP : 0u) | (split ? OS_SHARE : 0u) | (top ? OS_TOP : 0u);
+            return oc_smooth(M, L, what, T, t, rank, res, to);
+        }
+        // (level 0 leaves its last red half sweep to the r.z pass)
+        for (int sw = 0; sw < level_sweeps(l); sw++) {
+            const bool end = sw + 1 == level_sweeps(l), stop = up && end && l == 0, out = up && end && top;
+            sweep(l, 1, T.n, split && !stop);
+            if (stop) return;
+            T.sync();
+            if (!up && end) break;
+            sweep(l, 0, T.n, split && !out);
+            if (!(out && split)) T.sync();
+        }
+        if (!up) residual(l, res, T.n, to);
+    };
     {
         const OcLevel &L = S.lv[Q.lo];
         const float *gx = M.lv[Q.lo].x, *gb = M.lv[Q.lo].b;
-        for (int e = t; e < L.n + 2 * L.rp && L.n > 0; e += nt) {
-            const OcItem it(L, e, -1);
-            if (it.i < 0 || it.i >= L.nx) continue;
-            const int m = e - L.rp;
-            const bool own = m >= 0 && m < L.n;
+        const int n = L.n, rp = L.rp, all_ = n > 0 ? n + 2 * rp : 0, nx = L.nx, ny = L.ny, nz = L.nz;
+        float *const xs[2] = {L.x(0), L.x(1)}, *const bs[2] = {L.b(0), L.b(1)};
+        constexpr int U = 4;      // pairs in flight
+        for (int e0 = t; e0 < all_; e0 += U * nt) {
+            float xv[U][2], bv[U][2];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int k = 2 * it.p + h, c = ((it.i + it.j) & 1) ^ h;
-                if (k >= L.nz) continue;
-                const int cell = (it.i * L.ny + it.j) * L.nz + k;
-                L.x(c)[e] = __ldcg(gx + cell);
-                if (own) L.b(c)[m] = __ldcg(gb + cell);
+            for (int u = 0; u < U; u++) {
+                const OcItem it(L, min(e0 + u * nt, all_ - 1), -1);
+                const int i = max(0, min(it.i, nx - 1)), cell = (i * ny + it.j) * nz + 2 * it.p, two = 2 * it.p + 1 < nz;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    xv[u][h] = __ldcg(gx + cell + h * two);
+                    bv[u][h] = __ldcg(gb + cell + h * two);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int e = e0 + u * nt, m = e - rp;
+                if (e >= all_) break;
+                const OcItem it(L, e, -1);
+                if (it.i < 0 || it.i >= nx) continue;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int c = ((it.i + it.j) & 1) ^ h;
+                    if (2 * it.p + h >= nz) continue;
+                    xs[c][e] = xv[u][h];
+                    if (m >= 0 && m < n) bs[c][m] = bv[u][h];
+                }
             }
         }
-        oc_sync(all);      // a neighbour's first push must find its halo loaded
+        all.sync();        // a neighbour's first push must find its halo loaded
     }
-    // down: the split levels by the cluster, the others by block 0 (a level of
-    // at most 32 pairs by its first warp, the other warps skip its barriers)
+    // down: the split levels by the cluster, the others by block 0
     for (int l = Q.lo; l < last; l++) {
-        const bool split = l < Q.fb, solo = !split && S.lv[l].nx * S.lv[l].rp <= 32;
-        const OcGroup g = split ? all : (solo ? OC_WARP : OC_BLOCK);
-        const int n = solo ? 32 : nt;
-        if (!split && (rank != 0 || (solo && t >= 32))) break;
-        for (int sw = 0; sw < level_sweeps(l); sw++) {
-            if (sw > 0) {
-                sweep(l, 0, n, split);
-                oc_sync(g);
-            }
-            sweep(l, 1, n, split);
-            oc_sync(g);
-        }
+        const bool split = l < Q.fb;
+        const OcTeam T = team_of(l);
+        if (!split && (rank != 0 || t >= T.n)) break;
         if (split && l + 1 == Q.fb) {
-            residual(l, res0 + S.lv[l].p0 * S.lv[l].rp, n, 0);
-            oc_sync(all);
+            smooth(l, T, false, res0 + S.lv[l].p0 * S.lv[l].rp, 0);
+            T.sync();
             if (rank != 0) break;
             oc_coarse_rhs(S.lv[l], 0, res0, S.lv[l + 1], t, nt, 0, false);
             __syncthreads();
         } else {
             // (a split level's coarse planes have their children in the same block)
-            residual(l, red, n, rank);
-            oc_sync(split ? OC_BLOCK : g);
-            oc_coarse_rhs(S.lv[l], S.lv[l].p0, red, S.lv[l + 1], t, n, rank, split);
-            oc_sync(g);
+            smooth(l, T, false, red, rank);
+            if (split) __syncthreads();
+            else T.sync();
+            oc_coarse_rhs(S.lv[l], S.lv[l].p0, red, S.lv[l + 1], t, T.n, rank, split);
+            T.sync();
         }
     }
-    bool narrow = S.lv[last].nx * S.lv[last].rp <= 32;
+    const int coarsest = S.lv[last].nx * S.lv[last].rp;
     if (rank == 0) {
-        if (narrow) {
+        if (coarsest <= 32) {
             if (t < 32) oc_coarsest(M, S.lv[last], t);
-        } else {
+        } else if (t < team_of(last).n) {
+            const OcTeam T = team_of(last);
             for (int sw = 0; sw < kCoarsestSweeps; sw++)
                 for (int c = 1; c >= 0; c--) {
-                    sweep(last, c, nt, false);
-                    __syncthreads();
+                    sweep(last, c, T.n, false);
+                    T.sync();
                 }
         }
     }
     // up
     for (int l = last - 1; l >= Q.lo; l--) {
-        const bool split = l < Q.fb, solo = !split && S.lv[l].nx * S.lv[l].rp <= 32;
-        if (!split && rank != 0) continue;
-        const OcGroup g = split ? all : (solo ? OC_WARP : OC_BLOCK);
-        const int n = solo ? 32 : nt;
-        if (rank == 0 && narrow && !solo) __syncthreads();     // the warp's results to the whole block
-        narrow = solo;
-        if (solo && t >= 32) continue;
-        if (solo) __syncwarp();
+        const bool split = l < Q.fb;
+        const OcTeam T = team_of(l);
+        if (!split && (rank != 0 || t >= T.n)) continue;
+        // the coarser level's results to all who need them
+        if (!split || l + 1 == Q.fb) T.sync();
         if (split && l + 1 == Q.fb) {
             // from block 0, through a copy of the planes around this block's parents
-            oc_sync(all);
             const OcLevel &L = S.lv[l], &B = S.lv[Q.fb];
             const int first = max(0, (L.p0 - 1) >> L.sx), end = min(B.nx, ((L.p0 + L.np) >> L.sx) + 1);
             float *copy = oc_smem + Q.off_par;
@@ -455,22 +569,13 @@ __device__ __noinline__ void oc_vcycle(const PCGArgs &A, const OnchipPlan &Q, in
             __syncthreads();
             oc_prolong(L, B, Q.off_par, first, count, t, nt);
         } else {
-            oc_prolong(S.lv[l], S.lv[l + 1], -1, 0, 0, t, n);
+            oc_prolong(S.lv[l], S.lv[l + 1], -1, 0, 0, t, T.n);
         }
         // (a neighbour stores into the red halo, prolonged here, after the next
         // cluster barrier only)
-        oc_sync(split ? OC_BLOCK : g);
-        // level lo's last half sweep needs no halo; level 0 leaves its last red
-        // half sweep to the r.z pass
-        const bool top = l == Q.lo;
-        for (int sw = 0; sw < level_sweeps(l); sw++) {
-            const bool end = sw + 1 == level_sweeps(l);
-            sweep(l, 1, n, split && !(end && l == 0));
-            if (end && l == 0) break;
-            oc_sync(g);
-            sweep(l, 0, n, split && !(end && top));
-            if (!(split && end && top)) oc_sync(g);
-        }
+        if (split) __syncthreads();
+        else T.sync();
+        smooth(l, T, true, nullptr, rank);
     }
     __syncthreads();
     {
