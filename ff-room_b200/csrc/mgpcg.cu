@@ -643,12 +643,14 @@ struct GridGroup {
     __device__ static void finish() {}
 };
 
+constexpr int kMaxClusterCtas = 16;
+
 struct ClusterGroup {
     __device__ static int rank() { return (int)cooperative_groups::this_cluster().block_rank(); }
     __device__ static int size() { return (int)cooperative_groups::this_cluster().num_blocks(); }
-    __device__ static double (&slots())[2][4]
+    __device__ static double (&slots())[2][2][kMaxClusterCtas]
     {
-        __shared__ double s_slot[2][4];
+        __shared__ double s_slot[2][2][kMaxClusterCtas];
         return s_slot;
     }
     __device__ static int &parity()
@@ -661,35 +663,37 @@ struct ClusterGroup {
         if (threadIdx.x == 0) parity() = 0;
         __syncthreads();
     }
+    // (the barrier orders the cluster's global accesses as well as its shared ones)
     __device__ static bool sync(const PCGArgs &)
     {
-        __threadfence();
         cooperative_groups::this_cluster().sync();
         return true;
     }
-    // Deterministic: every block adds the blocks' partials in rank order.
-    // Two slot buffers alternate, so a block never overwrites a slot another
-    // block may still be reading (a cluster barrier separates the reuse).
+    // Deterministic: every block adds the blocks' partials in rank order, each
+    // partial handed to every block ahead of the barrier (read from the other
+    // blocks after it, one after another, they took 3 k cycles).  Two slot
+    // buffers alternate, so a block never overwrites a slot another block may
+    // still be reading (a cluster barrier separates the reuse).
     template <int NV>
     __device__ static bool allreduce(const PCGArgs &, double (&v)[NV], double *sh)
     {
         auto cl = cooperative_groups::this_cluster();
-        const int p = parity();
+        const int nb = (int)cl.num_blocks();
+        int p = 0;
         for (int a = 0; a < NV; a++) {
             const double t = block_sum(v[a], sh);
-            if (threadIdx.x == 0) slots()[p][a] = t;
+            if (a == 0) p = parity();
+            if (threadIdx.x < nb) cl.map_shared_rank(&slots()[p][a][0], threadIdx.x)[cl.block_rank()] = t;
         }
-        __threadfence();
         cl.sync();
-        const int nb = (int)cl.num_blocks();
         for (int a = 0; a < NV; a++) {
             double tot = 0.0;
-            for (int r = 0; r < nb; r++) tot += *cl.map_shared_rank(&slots()[p][a], r);
+#pragma unroll
+            for (int r = 0; r < kMaxClusterCtas; r++)
+                if (r < nb) tot += slots()[p][a][r];
             v[a] = tot;
         }
-        __syncthreads();
         if (threadIdx.x == 0) parity() = p ^ 1;
-        __syncthreads();
         return true;
     }
     // no block may leave while another can still read its shared memory
