@@ -1938,9 +1938,31 @@ unsigned split_blocks_level0(long long n)
     return (unsigned)std::max<long long>(1, std::min<long long>((n + 1023) / 1024, kSplitMaxBlocks));
 }
 
-// Grid sizes of the split solve's launches: two items (pairs or coarse
-// cells) per thread, so each block amortises its start-up over more work
-// (many rooms in one batched launch fill the GPU by their number).
+// Launch shape of the split solve's passes over one level (items: pairs or coarse
+// cells).  A large level takes two items per thread in blocks of 256, so each
+// block amortises its start-up; a level that cannot fill the GPU that way takes
+// one per thread in blocks of 128, which puts it on twice to four times as many
+// SMs (us per iteration: 315 k cells 112 -> 105, 1.0 M 159 -> 153, 7.9 M 522 -> 518;
+// with the line at 1.2 M cells instead of 400 k, 1.0 M 155).
+constexpr long long kSmallLevelCells = 400000;
+struct LevelShape {
+    unsigned blocks, threads;
+    LevelShape(const MGDev &M, int l, long long items)
+        : threads(M.lv[l].n <= kSmallLevelCells ? 128 : 256)
+    {
+        const long long per = threads == 128 ? 128 : 512;
+        blocks = (unsigned)std::max<long long>(1, (items + per - 1) / per);
+    }
+};
+
+LevelShape split_shape_pairs(const MGDev &M, int l)
+{
+    const MGLevel &L = M.lv[l];
+    return LevelShape(M, l, (long long)L.nx * L.ny * ((L.nz + 1) / 2));
+}
+
+// Grid sizes of the batched split solve's launches, two items per thread (many
+// rooms in one launch fill the GPU by their number).
 unsigned split_blocks_pairs(const MGDev &M, int l)
 {
     const MGLevel &L = M.lv[l];
@@ -2030,16 +2052,21 @@ int split_iteration(const PCGArgs &a, SplitState *ss, cudaStream_t bs, cudaGraph
         if (e != cudaSuccess && rc == FFR_OK) rc = cuda_fail(e, "split kernel launch");
         count_launch(1);
     };
+    auto smooth = [&](auto *kernel, int l, int color) {
+        const LevelShape sh = split_shape_pairs(M, l);
+        chk(launch_chained(kernel, sh.blocks, sh.threads, bs, 0, 0, a, ss, l, color));
+    };
     if (M.nlev > 1) {
         const int top = std::min(M.nlev_grid, M.nlev - 1);
         const int gdown = std::min(M.nlev_mid, top);
         for (int l = 0; l < gdown; l++) {
-            chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 1));
+            smooth(k_sp_smooth<false>, l, 1);
             for (int sw = 1; sw < level_sweeps(l); sw++) {
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 0));
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 1));
+                smooth(k_sp_smooth<false>, l, 0);
+                smooth(k_sp_smooth<false>, l, 1);
             }
-            chk(launch_chained(k_sp_restrict, split_blocks_cells(M, l + 1), 256, bs, 0, 0, a, ss, l));
+            const LevelShape sh(M, l + 1, M.lv[l + 1].n);
+            chk(launch_chained(k_sp_restrict, sh.blocks, sh.threads, bs, 0, 0, a, ss, l));
         }
         if (M.nlev_mid < top || M.nlev_grid < M.nlev) {
             const int ctas = mid_cluster_ctas();
@@ -2050,19 +2077,19 @@ int split_iteration(const PCGArgs &a, SplitState *ss, cudaStream_t bs, cudaGraph
                 chk(launch_chained(k_sp_mid, ctas, kMidThreads, bs, ctas, 0, a, ss, M.nlev_mid));
         }
         for (int l = gdown - 1; l >= 1; l--) {
-            chk(launch_chained(k_sp_smooth<true>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 1));
-            chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 0));
+            smooth(k_sp_smooth<true>, l, 1);
+            smooth(k_sp_smooth<false>, l, 0);
             for (int sw = 1; sw < level_sweeps(l); sw++) {
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 1));
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, l), 256, bs, 0, 0, a, ss, l, 0));
+                smooth(k_sp_smooth<false>, l, 1);
+                smooth(k_sp_smooth<false>, l, 0);
             }
         }
         if (M.nlev_grid >= 1) {
-            chk(launch_chained(k_sp_smooth<true>, split_blocks_pairs(M, 0), 256, bs, 0, 0, a, ss, 0, 1));
+            smooth(k_sp_smooth<true>, 0, 1);
             // the further sweeps; the last red half is k_sp_redpost's
             for (int sw = 1; sw < level_sweeps(0); sw++) {
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, 0), 256, bs, 0, 0, a, ss, 0, 0));
-                chk(launch_chained(k_sp_smooth<false>, split_blocks_pairs(M, 0), 256, bs, 0, 0, a, ss, 0, 1));
+                smooth(k_sp_smooth<false>, 0, 0);
+                smooth(k_sp_smooth<false>, 0, 1);
             }
         }
     }
