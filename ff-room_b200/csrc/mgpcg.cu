@@ -53,10 +53,20 @@ void build_mg_levels(const HostRoom &r, MGHost &out)
     int nx = r.g.nx, ny = r.g.ny, nz = r.g.nz;
     out.nx.push_back(nx); out.ny.push_back(ny); out.nz.push_back(nz);
     const double lx = r.g.lx, ly = r.g.ly, lz = r.g.lz;
-    while ((size_t)nx * ny * nz > (size_t)kCoarsestCells && (int)out.nx.size() < kMaxLevels) {
+    // (one level below the fine one at least: only its correction and the sweeps
+    // around it reach the fine level's black cells)
+    while (((size_t)nx * ny * nz > (size_t)kCoarsestCells || out.nx.size() == 1) && (int)out.nx.size() < kMaxLevels) {
         // axes to halve at this level
         const double hx = lx / nx, hy = ly / ny, hz = lz / nz;
-        const double hmin = std::min(hx, std::min(hy, hz));
+        double hmin = std::min(hx, std::min(hy, hz));
+        if (out.nx.size() == 1 && !(nx > 1 && hx < 2.0 * hmin) && !(ny > 1 && hy < 2.0 * hmin) &&
+            !(nz > 1 && hz < 2.0 * hmin)) {
+            // the smallest spacing is that of an axis of one cell: the others'
+            hmin = 1e300;
+            if (nx > 1) hmin = std::min(hmin, hx);
+            if (ny > 1) hmin = std::min(hmin, hy);
+            if (nz > 1) hmin = std::min(hmin, hz);
+        }
         const int sx = (nx > 1 && hx < 2.0 * hmin) ? 1 : 0;
         const int sy = (ny > 1 && hy < 2.0 * hmin) ? 1 : 0;
         const int sz = (nz > 1 && hz < 2.0 * hmin) ? 1 : 0;
@@ -1684,8 +1694,9 @@ int mg_upload(const HostRoom &r, const MGHost &h, const RoomDev &R, Arena &ar, H
 {
     const RoomGeom &g = r.g;
     M.nlev = (int)h.nx.size();
-    M.nlev_grid = 0;
-    for (int l = 0; l < M.nlev; l++)
+    // (the fine level has no explicit coefficients, which the levels of one block need)
+    M.nlev_grid = 1;
+    for (int l = 1; l < M.nlev; l++)
         if ((long long)h.nx[l] * h.ny[l] * h.nz[l] > kBlockLevelCells) M.nlev_grid = l + 1;
     // first level (>= 1) small enough for the one-cluster part of the split solve
     M.nlev_mid = 1;
