@@ -18,9 +18,10 @@
 //      Gauss-Seidel, kSmoothSweeps sweeps red then black before the coarse
 //      correction and black then red after it, so the V-cycle is a
 //      symmetric operator and CG applies.
-// The whole solve is one cooperative launch; levels larger than
-// kBlockLevelCells are swept by the whole grid between grid barriers, the
-// remaining small levels by block 0 alone.
+// The whole solve is one cooperative launch, one thread-block cluster or one
+// kernel per pass.  Levels larger than kBlockLevelCells are swept by the whole
+// group, the remaining small levels by block 0 alone; a cluster keeps the
+// levels that fit in its shared memory there (mgonchip.cuh).
 #include "mgpcg.cuh"
 
 #include <cooperative_groups.h>
@@ -1846,9 +1847,9 @@ template <class F> int allow_cluster(F *fn, size_t smem)
 
 // The finest level that fits: up to about 150 k cells on 16 blocks that is
 // level 0.  Per iteration with 16 blocks, the V-cycle in global memory and on
-// chip: 15 k cells (8 blocks) 103 -> 80 us, 52 k 142 -> 110, 92 k 159 -> 124,
-// 192 k (from level 1 on) 224 -> 201; the levels of at most 32 k cells below a
-// split solve (k_sp_mid) 70 -> 40 us.
+// chip: 15 k cells (8 blocks) 103 -> 59 us, 52 k 142 -> 94, 92 k 159 -> 111,
+// 192 k (from level 1 on) 224 -> 190; the levels of at most 32 k cells below a
+// split solve (k_sp_mid), cold caches, 70 -> 35 us at 315 k cells.
 bool plan_onchip(const MGDev &M, int ctas, int lo_min, size_t bytes, OnchipPlan &out)
 {
     // (a hierarchy that could not be coarsened to a block-sized level has no
