@@ -645,6 +645,7 @@ struct GridGroup {
     __device__ static int rank() { return blockIdx.x; }
     __device__ static int size() { return gridDim.x; }
     __device__ static void init() {}
+    __device__ static void ready() {}
     __device__ static bool sync(const PCGArgs &A) { return grid_barrier(A.gs); }
     template <int NV>
     __device__ static bool allreduce(const PCGArgs &A, double (&v)[NV], double *sh)
@@ -673,7 +674,11 @@ struct ClusterGroup {
     {
         if (threadIdx.x == 0) parity() = 0;
         __syncthreads();
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     }
+    // Before the first access to another block's shared memory: every block of
+    // the cluster runs (has passed init; the wait lies under the set-up).
+    __device__ static void ready() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
     // (the barrier orders the cluster's global accesses as well as its shared ones)
     __device__ static bool sync(const PCGArgs &)
     {
@@ -1114,6 +1119,7 @@ __device__ __forceinline__ void pcg_body(const PCGArgs &A)
     {
         double acc[2] = {0.0, 0.0};
         pass_init(A, t0, nth, acc);
+        G::ready();
         if (!G::template allreduce<2>(A, acc, sh)) { flags = FFR_FLAG_TIMEOUT; goto finish; }
         const double bnorm = sqrt(acc[0]);
         if (bnorm < 1e-15) goto finish;
