@@ -117,22 +117,22 @@ __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity)
 struct WaitLimit {
     unsigned spins = 0;
     unsigned long long t0 = 0;
-    __device__ __forceinline__ bool over(int *err)
+    __device__ __forceinline__ bool over(int *err, unsigned long long at_least = 0)
     {
         if ((++spins & 63u) != 0) return false;
         const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
-        if (now - t0 <= g_wait_limit_ns && !(err && *(volatile int *)err)) return false;
+        if (now - t0 <= max(g_wait_limit_ns, at_least) && !(err && *(volatile int *)err)) return false;
         if (err) atomicExch(err, 1);
         return true;
     }
 };
 
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity)
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, unsigned long long at_least = 0)
 {
     WaitLimit w;
     while (!bar_try(bar, parity))
-        if (w.over(nullptr)) return false;
+        if (w.over(nullptr, at_least)) return false;
     return true;
 }
 
@@ -219,18 +219,88 @@ struct ClusterLayout {
     }
 };
 
+// Pushes r of a block's `own` cells (in sr) to the blocks whose halo (srh) holds
+// it and counts it on their mbarrier bars[2].  By the last warp.
+__device__ __forceinline__ void push_halo(int own, int plane2, const double *sr, const double *srh,
+                                          const unsigned long long *bars)
+{
+    const int lane = threadIdx.x & 31, rank = blockIdx.x, base = rank * own;
+    if ((threadIdx.x >> 5) != kResThreads / 32 - 1 || lane >= (int)gridDim.x || lane == rank) return;
+    // own cells [lo, hi) that lie in block `lane`'s halo, before or after its cells
+    const int b0 = lane * own, b1 = b0 + own;
+    const int lo = lane > rank ? max(base, b0 - plane2) : base;
+    const int hi = lane > rank ? base + own : min(base + own, b1 + plane2);
+    if (lo >= hi) return;
+    const int at = lane > rank ? lo - (b0 - plane2) : plane2 + lo - b1;
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     peer_addr(smem_addr(srh + at), lane)),
+                 "r"(smem_addr(sr + lo - base)), "r"(8 * (hi - lo)), "r"(peer_addr(smem_addr(bars + 2), lane))
+                 : "memory");
+}
+
+// After a block of the cluster has given up: waits until every copy between the
+// blocks has arrived; true when they have.  A reduction ends once every block
+// has pushed, so all blocks are at the last one that any of them began (`seq`
+// counts them, `halos` the halos waited for) or the one before it.  Those
+// before it push what the others expect (the values no longer matter); then
+// all that was pushed is certain to arrive, and each block waits for what is
+// addressed to it.  Not inlined: inside the kernel it cost the four-cell form
+// 0.8 % (registers of the loop), as a function nothing.
+__device__ __noinline__ bool await_copies(int own, int plane2, int halo_bytes, unsigned seq, int halos, const double *sr,
+                                          const double *srh, double *parts, unsigned long long *bars, unsigned &s_seq)
+{
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, rank = blockIdx.x, blocks = gridDim.x;
+    const int V = own / kResGroup;
+    auto arrived = [&](unsigned q) {      // reduction q's partials
+        return bar_wait(smem_addr(bars + (q & 1)), ((q - 1) >> 1) & 1u, kBarrierTimeoutNs);
+    };
+    auto halo_arrived = [&](int h) { return bar_wait(smem_addr(bars + 2), (unsigned)h & 1u, kBarrierTimeoutNs); };
+    cooperative_groups::this_cluster().sync();
+    unsigned last = seq;
+    for (int b = 0; b < blocks; b++) {
+        unsigned v;
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(smem_addr(&s_seq), b)) : "memory");
+        last = max(last, v);
+    }
+    bool ok = seq == 0 || arrived(seq);
+    if (halos > 0) ok = halo_arrived(halos - 1) && ok;
+    __syncthreads();
+    if (last > seq) {
+        if (last & 1) push_halo(own, plane2, sr, srh, bars);
+        if (t == 0) bar_expect(smem_addr(bars + (last & 1)), 8 * V * blocks);
+        if (warp < V && lane < blocks) {
+            const int p = rank * V + warp;
+            push(peer_addr(smem_addr(parts + (last & 1) * (8 * kPadded) + (p >> 5) * kPadded + (p & 31)), lane), 0.0,
+                 peer_addr(smem_addr(bars + (last & 1)), lane));
+        }
+        ok = arrived(last) && ok;
+    }
+    if ((int)(last + 1) / 2 > halos) {
+        if (t == 0) bar_expect(smem_addr(bars + 2), halo_bytes);
+        ok = halo_arrived(halos) && ok;
+    }
+    return ok;
+}
+
 // Bound by the latency of an iteration's two reductions (about 900 cycles
 // each: staged values, one warp's tree per partial, st.async, mbarrier) and,
 // from K = 4 on, by shared-memory bandwidth (ten 8-byte accesses per cell).
 // Per iteration, k_cg before and this kernel: 6 000 cells 11.8 -> 2.7 us, 11.6 k
 // 12.2 -> 3.1, 25.7 k 12.1 -> 3.8, 50 k 13.1 -> 5.6.
-template <int K>
+//
+// Every wait is bounded.  A block whose wait runs out tells the others when
+// the cluster meets at the end, and then every copy still on its way is waited
+// for before a block leaves (below); the solve reports FFR_FLAG_TIMEOUT.
+//
+// ABSENT (self-test): the last block stays away from reduction A.absent_at.
+template <int K, bool ABSENT>
 __global__ void __launch_bounds__(kResThreads, 1) k_cg_cluster(CGArgs A, int nparts)
 {
     constexpr int OWN = K * kResThreads, V = OWN / kResGroup;   // cells and partials of a block
     constexpr int KW = K <= 2 ? K : 1;
     extern __shared__ __align__(16) double res_sm[];
     __shared__ __align__(8) unsigned long long s_bar[3];        // partials (two sets), halo
+    __shared__ unsigned s_gave_up, s_seq;
     if (A.st && A.st->halt) return;
     const RoomDev &R = A.R;
     const int nx = R.nx, ny = R.ny, nz = R.nz, n = R.n, plane = ny * nz;
@@ -244,6 +314,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_cluster(CGArgs A, int npa
     const int halo_bytes = 8 * (min(plane2, base) + min(plane2, (blocks - 1 - rank) * OWN));
 
     for (int a = t; a < lay.total; a += kResThreads) res_sm[a] = 0.0;
+    if (t == 0) s_gave_up = 0;
     __syncthreads();
     bool even = true;
     if (K > 2) {
@@ -259,34 +330,19 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_cluster(CGArgs A, int npa
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     cooperative_groups::this_cluster().sync();
 
-    unsigned seq = 0;                // reductions so far
-    int halos = 0, halos_sent = 0;   // halos received, halos pushed
+    unsigned seq = 0;                // reductions so far; the odd ones push a halo
+    int halos = 0;                   // halos received
     bool failed = false;             // a wait ran out
 
     // Sums what `put` staged (one value per own cell) over all cells;
     // with_halo also pushes r (in sr) to the blocks whose halo holds it.
     auto put = [&](int q, double v) { stage[(q * (kResThreads / 32) + warp) * kPadded + lane] = v; };
     auto reduce = [&](bool with_halo, double &total) -> bool {
+        if (ABSENT && rank == blocks - 1 && (int)seq + 1 == A.absent_at) return false;
         seq++;
         if (with_halo) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (with_halo) {
-            halos_sent++;
-            if (warp == kResThreads / 32 - 1 && lane < blocks && lane != rank) {
-                // own cells [lo, hi) that lie in block `lane`'s halo, before or after its cells
-                const int b0 = lane * OWN, b1 = b0 + OWN;
-                const int lo = lane > rank ? max(base, b0 - plane2) : base;
-                const int hi = lane > rank ? base + OWN : min(base + OWN, b1 + plane2);
-                if (lo < hi) {
-                    const int at = lane > rank ? lo - (b0 - plane2) : plane2 + lo - b1;
-                    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], "
-                                 "%2, [%3];" ::"r"(peer_addr(smem_addr(srh + at), lane)),
-                                 "r"(smem_addr(sr + lo - base)), "r"(8 * (hi - lo)),
-                                 "r"(peer_addr(smem_addr(&s_bar[2]), lane))
-                                 : "memory");
-                }
-            }
-        }
+        if (with_halo) push_halo(OWN, plane2, sr, srh, s_bar);
         const unsigned bar = smem_addr(&s_bar[seq & 1]);
         double *set = parts + (seq & 1) * (8 * kPadded);
         if (t == 0) bar_expect(bar, 8 * V * blocks);
@@ -418,14 +474,26 @@ finish:
         const int c = base + t + q * kResThreads;
         if (c < n) A.x[c] = x[q];
     }
-    // a halo still on its way here is waited for: no copy outlives the solve
-    if (halos_sent > halos && !(flags & FFR_FLAG_TIMEOUT)) {
+    // the halo that the last reduction pushed
+    failed = (flags & FFR_FLAG_TIMEOUT) != 0;
+    if (!failed && (seq & 1)) {
         if (t == 0) bar_expect(smem_addr(&s_bar[2]), halo_bytes);
-        if (!bar_wait(smem_addr(&s_bar[2]), (unsigned)halos & 1u)) flags |= FFR_FLAG_TIMEOUT;
+        failed = !bar_wait(smem_addr(&s_bar[2]), (unsigned)halos & 1u);
+        halos++;
+    }
+    // no block leaves while another may still write its shared memory, and a
+    // block that gave up says so to all
+    if (__syncthreads_or(failed) && t < blocks)
+        asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(peer_addr(smem_addr(&s_gave_up), t)) : "memory");
+    cooperative_groups::this_cluster().sync();
+    if (s_gave_up) {
+        if (t == 0) s_seq = seq;
+        const bool landed = await_copies(OWN, plane2, halo_bytes, seq, halos, sr, srh, parts, s_bar, s_seq);
+        if (ABSENT && !__syncthreads_and(landed) && t == 0) atomicExch(A.absent_lost, 1);
+        cooperative_groups::this_cluster().sync();
+        flags |= FFR_FLAG_TIMEOUT;
     }
     if (rank == 0 && t == 0) res_results(A, res, iters, flags);
-    // and no block leaves while another may still write its shared memory
-    cooperative_groups::this_cluster().sync();
 }
 
 // ----------------------------------------------------------------- grid
@@ -467,8 +535,11 @@ constexpr int kSlotWords = 2 * kMailboxes * 2 * kChunkBlocks;
 // each side of an exchange.  Per iteration, k_cg before and this kernel: 72 k
 // cells 14.2 -> 6.7 us, 123 k 15.2 -> 6.9.
 //
+// ABSENT (self-test): the last block stays away from reduction A.absent_at.
+//
 // `words`: the tagged halves of r, {lo, hi} per cell; `slots`: those of the
 // block sums, two sets of kMailboxes x 128, then the error word.
+template <bool ABSENT>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_cg_chunks(CGArgs A, unsigned long long *words, unsigned long long *slots, int nparts)
 {
@@ -504,6 +575,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     // Sums val over all cells; with a tag also collects the halo's r
     // published under it, while the block sums travel.
     auto reduce = [&](const double (&val)[K], unsigned tag, double &total) -> bool {
+        if (ABSENT && block == kChunkBlocks - 1 && (int)seq + 1 == A.absent_at) return false;
         seq++;
 #pragma unroll
         for (int q = 0; q < K; q++) stage[(q * (kResThreads / 32) + warp) * kPadded + lane] = val[q];
@@ -663,9 +735,10 @@ namespace {
 
 template <int K> int launch_cluster(const CGArgs &a, int nparts, cudaStream_t s)
 {
+    auto *fn = a.absent_at ? k_cg_cluster<K, true> : k_cg_cluster<K, false>;
     const size_t smem = 8 * (size_t)ClusterLayout(K, a.R.nx, a.R.ny, a.R.nz).total;
-    FFR_CUDA(cudaFuncSetAttribute(k_cg_cluster<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    FFR_CUDA(cudaFuncSetAttribute(k_cg_cluster<K>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     const unsigned blocks = cdiv(nparts, K * kResThreads / kResGroup);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
@@ -679,21 +752,22 @@ template <int K> int launch_cluster(const CGArgs &a, int nparts, cudaStream_t s)
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FFR_CUDA(cudaLaunchKernelEx(&cfg, k_cg_cluster<K>, a, nparts));
+    FFR_CUDA(cudaLaunchKernelEx(&cfg, fn, a, nparts));
     count_launch(1);
     return FFR_OK;
 }
 
 int launch_chunks(const CGArgs &a, int nparts, cudaStream_t s)
 {
+    auto *fn = a.absent_at ? k_cg_chunks<true> : k_cg_chunks<false>;
     const size_t smem = 8 * (size_t)ChunkLayout(a.R.nz).total;
-    FFR_CUDA(cudaFuncSetAttribute(k_cg_chunks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     unsigned long long *words = reinterpret_cast<unsigned long long *>(a.da);
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(a.ad);
     // the block sums' numbers and the error word start at zero
     FFR_CUDA(cudaMemsetAsync(slots, 0, 8 * (kSlotWords + 1), s));
     void *args[] = {(void *)&a, &words, &slots, &nparts};
-    FFR_CUDA(cudaLaunchCooperativeKernel((void *)k_cg_chunks, dim3(kChunkBlocks), dim3(kResThreads), args, smem, s));
+    FFR_CUDA(cudaLaunchCooperativeKernel((void *)fn, dim3(kChunkBlocks), dim3(kResThreads), args, smem, s));
     count_launch(1);
     return FFR_OK;
 }

@@ -2592,6 +2592,44 @@ int ffr_poisson_solve_dev(ffr_poisson *s, const double *rhs_dev, double *p_dev, 
     return FFR_OK;
 }
 
+int ffr_poisson_selftest_wait(ffr_poisson *s, const double *rhs, int reduction, int *lost, double *elapsed_ms)
+{
+    if (!s || !rhs || !lost || !elapsed_ms) return fail(FFR_EINVAL, "NULL argument");
+    if (reduction < 1 || reduction > 1000) return fail(FFR_EINVAL, "reduction must be in [1, 1000]");
+    cudaStream_t st = s->stream;
+    FFR_CUDA(cudaMemcpyAsync(s->b_tmp, rhs, 8 * s->room.g.n, cudaMemcpyHostToDevice, st));
+    FFR_CUDA(cudaMemsetAsync(s->gs, 0, sizeof(GridSync), st));
+    CGArgs ca{};
+    ca.R = s->R;
+    ca.rhs = s->b_tmp;
+    ca.x = s->x_tmp; ca.r = s->r; ca.da = s->da; ca.db = s->db; ca.ad = s->ad;
+    ca.max_iter = s->max_iter; ca.tol = s->tol;
+    ca.out_res = s->res; ca.out_iters = s->iters; ca.out_flags = s->flags;
+    ca.absent_at = reduction;
+    ca.absent_lost = &s->gs->err;
+    cudaEvent_t ev[2];
+    FFR_CUDA(cudaEventCreate(&ev[0]));
+    FFR_CUDA(cudaEventCreate(&ev[1]));
+    bool taken = false;
+    FFR_CUDA(cudaEventRecord(ev[0], st));
+    int rc = s->blocks == cdiv(s->R.n, kThreads) ? launch_cg_resident(ca, st, &taken) : FFR_OK;
+    int fl = 0;
+    float ms = 0.0f;
+    if (!rc && !taken) rc = fail(FFR_ENOTSUP, "this room's solve has no on-chip form");
+    if (!rc) {
+        FFR_CUDA(cudaEventRecord(ev[1], st));
+        FFR_CUDA(cudaMemcpyAsync(&fl, s->flags, 4, cudaMemcpyDeviceToHost, st));
+        FFR_CUDA(cudaMemcpyAsync(lost, &s->gs->err, 4, cudaMemcpyDeviceToHost, st));
+        FFR_CUDA(cudaStreamSynchronize(st));
+        FFR_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+        *elapsed_ms = ms;
+        if (fl & FFR_FLAG_TIMEOUT) rc = fail(FFR_ETIMEDOUT, "self-test wait gave up at the wait limit");
+    }
+    cudaEventDestroy(ev[0]);
+    cudaEventDestroy(ev[1]);
+    return rc;
+}
+
 int ffr_poisson_solve(ffr_poisson *s, const double *rhs, double *p, double *residual,
                       int *iterations)
 {

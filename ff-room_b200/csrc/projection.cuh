@@ -71,6 +71,10 @@ struct CGArgs {
     double *out_res;
     int *out_iters;
     int *out_flags;
+    // self-test of the on-chip form's waits: the last block stays away from
+    // this reduction (0: none); *absent_lost is set where a copy did not arrive
+    int absent_at;
+    int *absent_lost;
 };
 
 // The reference's unpreconditioned CG as one cooperative launch

@@ -123,6 +123,7 @@ def lib():
             "ffr_poisson_solve_dev": ([vp, vp, vp, vp, _dp, C.POINTER(C.c_int)], C.c_int),
             "ffr_poisson_solve": ([vp, _dp, _dp, _dp, C.POINTER(C.c_int)], C.c_int),
             "ffr_poisson_apply": ([vp, _dp, _dp], C.c_int),
+            "ffr_poisson_selftest_wait": ([vp, _dp, C.c_int, C.POINTER(C.c_int), _dp], C.c_int),
             "ffr_lbm_create": ([C.POINTER(RoomDesc), C.c_double, C.c_int, C.c_double, C.c_double, C.c_int,
                                 C.POINTER(Fields), C.POINTER(vp)], C.c_int),
             "ffr_lbm_destroy": ([vp], C.c_int),
@@ -478,6 +479,13 @@ class PoissonHandle:
                                           C.c_void_p(stream) if stream else None, C.byref(res),
                                           C.byref(it)))
         return res.value, it.value
+
+    def selftest_wait(self, rhs, reduction: int):
+        """(status, copies lost, elapsed_ms) of a solve whose last block stays away from a reduction."""
+        rhs = np.ascontiguousarray(rhs, dtype=np.float64)
+        lost, ms = C.c_int(-1), C.c_double(0.0)
+        st = lib().ffr_poisson_selftest_wait(self.h, rhs.ctypes.data_as(_dp), int(reduction), C.byref(lost), C.byref(ms))
+        return st, lost.value, ms.value
 
     def apply(self, x):
         x = np.ascontiguousarray(x, dtype=np.float64)

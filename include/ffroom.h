@@ -48,7 +48,7 @@ const char *ffr_status_string(int status);
 /* Detail of the most recent failure on the calling thread ("" if none). */
 const char *ffr_last_error(void);
 /* Upper bound of every bounded device-side wait (the grid barriers of the
- * persistent solves), in seconds on the current device; 0 restores the
+ * persistent solves, the exchanges of the on-chip one), in seconds on the current device; 0 restores the
  * default of 4 s.  For tests of the failure path; no counterpart in the
  * reference. */
 int ffr_set_device_wait_limit(double seconds);
@@ -375,6 +375,16 @@ int ffr_poisson_solve_dev(ffr_poisson *s, const double *rhs_dev, double *p_dev,
 /* The same on host buffers (uploads rhs, downloads p). */
 int ffr_poisson_solve(ffr_poisson *s, const double *rhs, double *p,
                       double *residual, int *iterations);
+
+/* Self-test of the waits of the on-chip solve (rooms of at most 131 072
+ * cells): a solve whose last thread block stays away from one reduction
+ * (1, 2, ...), so that the others' waits run out at the wait limit.  Returns
+ * FFR_ETIMEDOUT with the kernel's duration; *lost is 0 when every copy
+ * between blocks had arrived before a block left.  FFR_OK when the solve
+ * ended before that reduction.  The handle stays usable.  No counterpart in
+ * the reference. */
+int ffr_poisson_selftest_wait(ffr_poisson *s, const double *rhs, int reduction,
+                              int *lost, double *elapsed_ms);
 
 /* PoissonSolver::apply_laplacian (PoissonSolver.cpp:22-91) on host buffers. */
 int ffr_poisson_apply(ffr_poisson *s, const double *x, double *ax);
