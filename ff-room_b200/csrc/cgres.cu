@@ -733,11 +733,40 @@ FFR_DEFINE_WAIT_LIMIT_SETTER(set_wait_limit_cgres)
 
 namespace {
 
+// Shared memory beside the dynamic part (a kernel's static arrays).
+constexpr int kResStatic = 256;
+
+struct ResLimits {
+    int sms = 0, smem = 0;       // SMs, dynamic shared memory of one block at most
+    ResLimits()
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        smem -= kResStatic;
+    }
+};
+const ResLimits &limits()
+{
+    static const ResLimits l;
+    return l;
+}
+
+// Lets a kernel take all of the shared memory.  (The limit is one value per
+// kernel and process: set to what each room needs, a launch of a smaller room
+// in another thread would lower it between a larger one's call and its launch.)
+template <class F> int allow_smem(F *fn)
+{
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limits().smem));
+    return FFR_OK;
+}
+
 template <int K> int launch_cluster(const CGArgs &a, int nparts, cudaStream_t s)
 {
     auto *fn = a.absent_at ? k_cg_cluster<K, true> : k_cg_cluster<K, false>;
     const size_t smem = 8 * (size_t)ClusterLayout(K, a.R.nx, a.R.ny, a.R.nz).total;
-    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(fn)) return rc;
     FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     const unsigned blocks = cdiv(nparts, K * kResThreads / kResGroup);
     cudaLaunchConfig_t cfg = {};
@@ -761,7 +790,7 @@ int launch_chunks(const CGArgs &a, int nparts, cudaStream_t s)
 {
     auto *fn = a.absent_at ? k_cg_chunks<true> : k_cg_chunks<false>;
     const size_t smem = 8 * (size_t)ChunkLayout(a.R.nz).total;
-    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(fn)) return rc;
     unsigned long long *words = reinterpret_cast<unsigned long long *>(a.da);
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(a.ad);
     // the block sums' numbers and the error word start at zero
@@ -776,18 +805,12 @@ int launch_chunks(const CGArgs &a, int nparts, cudaStream_t s)
 
 int launch_cg_resident(const CGArgs &a, cudaStream_t s, bool *taken)
 {
-    static int sms = 0, smem_max = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
+    const int smem_max = limits().smem;
     const RoomDev &R = a.R;
     const int nparts = (int)cdiv(R.n, kResGroup);
     auto cluster_fits = [&](int K) {
         return nparts <= kResClusterCtas * (K * kResThreads / kResGroup) && (long long)R.ny * R.nz < smem_max &&
-               8 * ClusterLayout(K, R.nx, R.ny, R.nz).total + 256 <= smem_max;
+               8 * ClusterLayout(K, R.nx, R.ny, R.nz).total <= smem_max;
     };
     // The smallest number of cells per thread that fits a cluster: the grid
     // form takes 6.8-7.0 us per iteration at any size, the cluster form 2.7 us
@@ -798,8 +821,8 @@ int launch_cg_resident(const CGArgs &a, cudaStream_t s, bool *taken)
     if (cluster_fits(4)) return launch_cluster<4>(a, nparts, s);
     if (cluster_fits(8)) return launch_cluster<8>(a, nparts, s);
     // r's words (16 bytes per cell) take both direction arrays, the slots A.ad
-    if (nparts <= kChunkMaxParts && sms >= kChunkBlocks && a.db - a.da >= R.n && R.n > kSlotWords &&
-        R.nz < smem_max / 128 && 8 * ChunkLayout(R.nz).total + 256 <= smem_max)
+    if (nparts <= kChunkMaxParts && limits().sms >= kChunkBlocks && a.db - a.da >= R.n && R.n > kSlotWords &&
+        R.nz < smem_max / 128 && 8 * ChunkLayout(R.nz).total <= smem_max)
         return launch_chunks(a, nparts, s);
     *taken = false;
     return FFR_OK;
