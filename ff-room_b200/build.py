@@ -20,7 +20,7 @@ CSRC = os.path.join(PKG, "csrc")
 INC = os.path.join(ROOT, "include")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 CUDA_SOURCES = ["room.cu", "projection.cu", "cgres.cu", "mgpcg.cu", "lbm.cu", "noalloc.cu", "server.cu"]
-HEADERS = ["common.cuh", "projection.cuh", "mgpcg.cuh", "mgonchip.cuh"]
+HEADERS = ["forms.h", "common.cuh", "projection.cuh", "mgpcg.cuh", "mgonchip.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 LIB = os.path.join(PKG, "libffroom_cuda.so")

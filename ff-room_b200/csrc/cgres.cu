@@ -22,6 +22,7 @@
 // Every sum is formed in k_cg's order (the 256 cells of a partial as its
 // blocks add them, the partials as its last arriver adds them), so the
 // results are bit-identical to k_cg's.
+#include "forms.h"
 #include "projection.cuh"
 
 #include <cooperative_groups.h>
@@ -29,11 +30,6 @@
 #include <algorithm>
 
 namespace ffr {
-
-constexpr int kResThreads = 512;
-constexpr int kResGroup = 256;               // cells of one partial (a k_cg block)
-constexpr int kResClusterCtas = 16;
-constexpr int kPadded = 36;                  // 32 values and 4 of padding (bank offset between groups)
 
 // A double as two 8-byte words {number, half} side by side; each word is
 // written and read whole.
@@ -197,27 +193,6 @@ __device__ __forceinline__ void res_results(const CGArgs &A, double res, int ite
 }
 
 // --------------------------------------------------------- one cluster
-
-__host__ __device__ constexpr int even_up(int v) { return (v + 1) & ~1; }
-
-// Shared memory of one block, in doubles.  Halos are padded to an even
-// number of cells at their outer end: a bulk copy moves 16-byte units.
-struct ClusterLayout {
-    int plane2;                              // cells of one halo side, padded
-    int dir, halo, own_r, stage, parts, table, total;
-    __host__ __device__ ClusterLayout(int K, int nx, int ny, int nz)
-    {
-        const int own = K * kResThreads;
-        plane2 = even_up(ny * nz);
-        dir = 0;                                        // direction: halo, own cells, halo
-        halo = dir + own + 2 * plane2;                  // r of the two halos
-        own_r = halo + 2 * plane2;                      // r of the own cells
-        stage = own_r + own;                            // one value per own cell
-        parts = stage + own / 32 * kPadded;             // two sets of 256 partials
-        table = parts + 2 * 8 * kPadded;
-        total = table + (K > 2 ? 2 * (nx + ny + nz) : 0);   // stencil scales (else in registers)
-    }
-};
 
 // Pushes r of a block's `own` cells (in sr) to the blocks whose halo (srh) holds
 // it and counts it on their mbarrier bars[2].  By the last warp.
@@ -501,34 +476,10 @@ finish:
 // The partials p, p + 256 and their partners 16 further on meet first in the
 // summation tree, so one block takes these four chunks of 256 cells and hands
 // out one value: 128 blocks, 128 values.
-constexpr int kChunks = 4, kChunkBlocks = 128;
-constexpr int kChunkMaxParts = 512;
 __device__ __forceinline__ int chunk_of(int block, int v)
 {
     return (block >> 4) * 32 + (block & 15) + 16 * (v >> 1) + 256 * (v & 1);
 }
-
-// Shared memory of one block, in doubles.  Each chunk keeps the direction on
-// three windows: its cells with nz more on either side, and the 256 cells
-// one plane before and one after.
-struct ChunkLayout {
-    int window, nhalo, dir, halo, at, stage, total;
-    __host__ __device__ ChunkLayout(int nz)
-    {
-        window = 3 * kResGroup + 2 * nz;
-        nhalo = kChunks * (2 * kResGroup + 2 * nz);
-        dir = 0;
-        halo = dir + kChunks * window;              // r of the halo cells, in window order
-        at = halo + nhalo;                          // their places in the windows and their cells
-        stage = at + nhalo;
-        total = stage + kChunks * 8 * kPadded;
-    }
-};
-
-// The block sums are handed out in kMailboxes copies: 128 blocks polling one
-// copy delay the stores to it (7.3k cycles per exchange; 2.9k with 16).
-constexpr int kMailboxes = 16;
-constexpr int kSlotWords = 2 * kMailboxes * 2 * kChunkBlocks;
 
 // Bound by the L2 round trips of the two exchanges (about 3 k cycles each of
 // 13 k per iteration).  Fences instead of numbered words cost 2-3 k cycles on
@@ -762,13 +713,27 @@ template <class F> int allow_smem(F *fn)
     return FFR_OK;
 }
 
+template <class F> int allow_cluster(F *fn)
+{
+    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return allow_smem(fn);
+}
+
+// Whether the device holds a cluster of `blocks` blocks of this form at once
+// (with all of the shared memory, whatever the room needs of it).
+template <int K> bool placeable(int blocks)
+{
+    static ClusterCheck check;
+    if (allow_cluster(k_cg_cluster<K, false>)) return false;
+    return check((const void *)k_cg_cluster<K, false>, blocks, kResThreads, (size_t)limits().smem);
+}
+
 template <int K> int launch_cluster(const CGArgs &a, int nparts, cudaStream_t s)
 {
     auto *fn = a.absent_at ? k_cg_cluster<K, true> : k_cg_cluster<K, false>;
     const size_t smem = 8 * (size_t)ClusterLayout(K, a.R.nx, a.R.ny, a.R.nz).total;
-    if (int rc = allow_smem(fn)) return rc;
-    FFR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    const unsigned blocks = cdiv(nparts, K * kResThreads / kResGroup);
+    if (int rc = allow_cluster(fn)) return rc;
+    const unsigned blocks = (unsigned)cluster_blocks(a.R.n, K);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kResThreads);
@@ -805,26 +770,20 @@ int launch_chunks(const CGArgs &a, int nparts, cudaStream_t s)
 
 int launch_cg_resident(const CGArgs &a, cudaStream_t s, bool *taken)
 {
-    const int smem_max = limits().smem;
     const RoomDev &R = a.R;
     const int nparts = (int)cdiv(R.n, kResGroup);
-    auto cluster_fits = [&](int K) {
-        return nparts <= kResClusterCtas * (K * kResThreads / kResGroup) && (long long)R.ny * R.nz < smem_max &&
-               8 * ClusterLayout(K, R.nx, R.ny, R.nz).total <= smem_max;
-    };
-    // The smallest number of cells per thread that fits a cluster: the grid
-    // form takes 6.8-7.0 us per iteration at any size, the cluster form 2.7 us
-    // at 6 k cells to 5.9 us at 64 k, on 16 SMs instead of 128.
-    *taken = true;
-    if (cluster_fits(1)) return launch_cluster<1>(a, nparts, s);
-    if (cluster_fits(2)) return launch_cluster<2>(a, nparts, s);
-    if (cluster_fits(4)) return launch_cluster<4>(a, nparts, s);
-    if (cluster_fits(8)) return launch_cluster<8>(a, nparts, s);
-    // r's words (16 bytes per cell) take both direction arrays, the slots A.ad
-    if (nparts <= kChunkMaxParts && limits().sms >= kChunkBlocks && a.db - a.da >= R.n && R.n > kSlotWords &&
-        R.nz < smem_max / 128 && 8 * ChunkLayout(R.nz).total <= smem_max)
-        return launch_chunks(a, nparts, s);
-    *taken = false;
+    const int form = cg_form(R.nx, R.ny, R.nz, limits().smem, limits().sms, a.db - a.da >= R.n, [](int K, int blocks) {
+        return K == 1 ? placeable<1>(blocks)
+                      : (K == 2 ? placeable<2>(blocks) : (K == 4 ? placeable<4>(blocks) : placeable<8>(blocks)));
+    });
+    *taken = form != CG_GRID;
+    switch (form) {
+    case 1: return launch_cluster<1>(a, nparts, s);
+    case 2: return launch_cluster<2>(a, nparts, s);
+    case 4: return launch_cluster<4>(a, nparts, s);
+    case 8: return launch_cluster<8>(a, nparts, s);
+    case CG_CHUNKS: return launch_chunks(a, nparts, s);
+    }
     return FFR_OK;
 }
 

@@ -9,6 +9,7 @@
 #include "ffroom.h"
 
 #include <algorithm>
+#include <atomic>
 #include <thread>
 #include <vector>
 
@@ -312,6 +313,36 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *slot, doub
 }
 
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
+
+// Whether the device can hold a cluster of `ctas` (1 to 16) blocks of one
+// kernel at once: asked of the driver once per size, from any thread.  (The
+// kernel's attributes must allow the size and the shared memory.)
+struct ClusterCheck {
+    std::atomic<signed char> known[17] = {};      // 0: not asked yet, 1: yes, -1: no
+    bool operator()(const void *fn, int ctas, unsigned threads, size_t smem)
+    {
+        if (ctas < 1 || ctas > 16) return false;
+        if (const int k = known[ctas].load()) return k > 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)ctas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        known[ctas].store(clusters > 0 ? 1 : -1);
+        return clusters > 0;
+    }
+};
 
 // Event-pair timing of kernel groups on one stream (host side).
 struct GroupTimer {
