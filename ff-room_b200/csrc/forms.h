@@ -99,4 +99,20 @@ int cg_form(int nx, int ny, int nz, int smem, int sms, bool pair, Place placeabl
     return CG_GRID;
 }
 
+// ------------------------- coarse levels of the split solve (mgpcg.cu)
+
+// One cluster: the largest of 16 and 8 blocks (16 needs the non-portable
+// cluster size) that the device can place; onchip: also with the levels in its
+// shared memory.  placeable(onchip, ctas) asks for either kernel.
+struct MidForm {
+    int ctas;
+    bool onchip;
+};
+template <class Place> MidForm mid_form(Place placeable)
+{
+    for (int ctas : {16, 8})
+        if (placeable(false, ctas)) return {ctas, placeable(true, ctas)};
+    return {1, placeable(true, 1)};
+}
+
 }  // namespace ffr

@@ -22,6 +22,7 @@
 // kernel per pass.  Levels larger than kBlockLevelCells are swept by the whole
 // group, the remaining small levels by block 0 alone; a cluster keeps the
 // levels that fit in its shared memory there (mgonchip.cuh).
+#include "forms.h"
 #include "mgpcg.cuh"
 
 #include <cooperative_groups.h>
@@ -1849,6 +1850,18 @@ template <class F> int allow_cluster(F *fn, size_t smem)
     return FFR_OK;
 }
 
+// Whether the device holds a cluster of `ctas` blocks of an on-chip kernel at
+// once (with kOnchipBytes, whatever the plan needs of them); where it does not,
+// the form in global memory runs.
+template <class F> bool onchip_placeable(F *fn, ClusterCheck &check, int ctas, unsigned threads)
+{
+    if (allow_cluster(fn, kOnchipBytes)) {
+        cudaGetLastError();
+        return false;
+    }
+    return check((const void *)fn, ctas, threads, kOnchipBytes);
+}
+
 }  // namespace
 
 // The finest level that fits: up to about 150 k cells on 16 blocks that is
@@ -1910,8 +1923,10 @@ bool plan_onchip(const MGDev &M, int ctas, int lo_min, size_t bytes, OnchipPlan 
 int launch_pcg_cluster(const PCGArgs &a0, cudaStream_t s, int ctas)
 {
     PCGArgs a = a0;
-    const bool onchip = plan_onchip(a.M, ctas, 0, kOnchipBytes, a.Q);
-    auto *fn = onchip ? k_pcg<ClusterGroup, kClusterThreads, true> : k_pcg<ClusterGroup, kClusterThreads, false>;
+    static ClusterCheck check;
+    auto *chip = k_pcg<ClusterGroup, kClusterThreads, true>;
+    const bool onchip = plan_onchip(a.M, ctas, 0, kOnchipBytes, a.Q) && onchip_placeable(chip, check, ctas, kClusterThreads);
+    auto *fn = onchip ? chip : k_pcg<ClusterGroup, kClusterThreads, false>;
     if (int rc = allow_cluster(fn, onchip)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
@@ -1993,34 +2008,18 @@ unsigned split_blocks_cells(const MGDev &M, int l)
     return (unsigned)std::max<long long>(1, ((long long)M.lv[l].n + 511) / 512);
 }
 
-// Cluster size of k_sp_mid: the largest of 16 and 8 blocks that the device
-// can co-schedule (16 needs the non-portable cluster-size attribute).
-int mid_cluster_ctas()
+// The split solve's cluster for the coarse levels on this device.
+MidForm mid_cluster()
 {
-    static int ctas = 0;
-    if (ctas) return ctas;
-    cudaFuncSetAttribute(k_sp_mid, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (allow_cluster(k_sp_mid_onchip, kOnchipBytes)) cudaGetLastError();
-    for (int want : {16, 8}) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)want);
-        cfg.blockDim = dim3(kMidThreads);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)want;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, k_sp_mid, &cfg) == cudaSuccess && nclusters > 0) {
-            ctas = want;
-            return ctas;
-        }
-        cudaGetLastError();
-    }
-    ctas = 1;
-    return ctas;
+    static const MidForm form = [] {
+        ClusterCheck plain, chip;
+        if (allow_cluster(k_sp_mid, 0)) cudaGetLastError();
+        return mid_form([&](bool onchip, int ctas) {
+            return onchip ? onchip_placeable(k_sp_mid_onchip, chip, ctas, kMidThreads)
+                          : plain((const void *)k_sp_mid, ctas, kMidThreads, 0);
+        });
+    }();
+    return form;
 }
 
 // Kernels one PCG iteration of the split solve runs (the body below).
@@ -2087,9 +2086,10 @@ int split_iteration(const PCGArgs &a, SplitState *ss, cudaStream_t bs, cudaGraph
             chk(launch_chained(k_sp_restrict, sh.blocks, sh.threads, bs, 0, 0, a, ss, l));
         }
         if (M.nlev_mid < top || M.nlev_grid < M.nlev) {
-            const int ctas = mid_cluster_ctas();
+            const MidForm mid = mid_cluster();
+            const int ctas = mid.ctas;
             PCGArgs am = a;
-            if (plan_onchip(M, ctas, M.nlev_mid, kOnchipBytes, am.Q) && am.Q.lo == M.nlev_mid)
+            if (mid.onchip && plan_onchip(M, ctas, M.nlev_mid, kOnchipBytes, am.Q) && am.Q.lo == M.nlev_mid)
                 chk(launch_chained(k_sp_mid_onchip, ctas, kMidThreads, bs, ctas, 4 * (size_t)am.Q.floats, am, ss));
             else
                 chk(launch_chained(k_sp_mid, ctas, kMidThreads, bs, ctas, 0, a, ss, M.nlev_mid));
@@ -2509,7 +2509,9 @@ int batch_split_solve(BatchSplit &B, cudaStream_t s, int max_iter)
 int launch_batch_cluster(BatchSplit &B, cudaStream_t s, int ctas)
 {
     if (B.nrooms == 0) return FFR_OK;
-    const bool onchip = B.cluster_floats > 0;
+    static ClusterCheck check;
+    const bool onchip =
+        B.cluster_floats > 0 && onchip_placeable(k_bpcg_cluster<true>, check, ctas, kClusterThreads);
     auto *fn = onchip ? k_bpcg_cluster<true> : k_bpcg_cluster<false>;
     if (int rc = allow_cluster(fn, onchip)) return rc;
     k_bsp_extrapolate<<<B.nb_cells0, 256, 0, s>>>(B.D, B.cells0);
@@ -2517,7 +2519,7 @@ int launch_batch_cluster(BatchSplit &B, cudaStream_t s, int ctas)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(B.nrooms * ctas));
     cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = 4 * (size_t)B.cluster_floats;
+    cfg.dynamicSmemBytes = onchip ? 4 * (size_t)B.cluster_floats : 0;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

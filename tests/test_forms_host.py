@@ -11,9 +11,16 @@ from conftest import PKG
 
 SRC = r"""
 #include <cstdio>
+#include <cstdlib>
 #include "forms.h"
-int main()
+int main(int argc, char **argv)
 {
+    if (argc == 3) {     // most blocks of the plain and of the on-chip kernel that can be placed
+        const int most[2] = {std::atoi(argv[1]), std::atoi(argv[2])};
+        const ffr::MidForm f = ffr::mid_form([&](bool onchip, int ctas) { return ctas <= most[onchip]; });
+        std::printf("%d %d\n", f.ctas, (int)f.onchip);
+        return 0;
+    }
     int nx, ny, nz, smem, sms, pair, most;
     while (std::scanf("%d %d %d %d %d %d %d", &nx, &ny, &nz, &smem, &sms, &pair, &most) == 7)
         std::printf("%d\n", ffr::cg_form(nx, ny, nz, smem, sms, pair != 0, [=](int, int blocks) { return blocks <= most; }));
@@ -58,3 +65,10 @@ def test_the_grid_form_needs_its_blocks_and_its_scratch(program):
     assert ask(program, 80, 64, 24, SMEM, 127, 1, 16) == GRID
     assert ask(program, 80, 64, 24, SMEM, SMS, 0, 16) == GRID
     assert ask(program, 80, 64, 24, 70000, SMS, 1, 16) == GRID
+
+
+@pytest.mark.parametrize("plain,chip,want", [(16, 16, (16, 1)), (16, 15, (16, 0)), (15, 15, (8, 1)), (8, 0, (8, 0)), (7, 7, (1, 1)),
+                                             (0, 0, (1, 0))])
+def test_coarse_levels(program, plain, chip, want):
+    out = subprocess.run([program, str(plain), str(chip)], text=True, capture_output=True, check=True).stdout
+    assert tuple(map(int, out.split())) == want
