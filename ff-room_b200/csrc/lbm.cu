@@ -155,7 +155,7 @@ template <> struct Store<2> {
 
 // Per-cell flags of the step kernel (besides the cell type in bits 0-1).
 enum : uint8_t { LF_OPEN = 4,    // all 18 neighbours in the domain and not SOLID
-                 LF_REMAP = 8 }; // OUTFLOW cell whose populations come from another cell
+                 LF_REMAP = 8 }; // in the remap list: stepped by step_remapped
 
 struct LbmDev {
     int nx, ny, nz, n, nu, nv, nw;
@@ -381,7 +381,10 @@ __device__ __forceinline__ void collide_cell(const LbmDev &L, int o, unsigned t,
 
 // The step of the re-mapped OUTFLOW cells i, i + stride, ... of the list: their
 // post-stream populations are those of another cell o (gathered as that cell
-// gathers its own), from there on the cell's own step.
+// gathers its own), from there on the cell's own step.  In the narrow modes the
+// list also holds the INFLOW cells without a fan, as their own source: what
+// arrives there stays as it is, and collide_pair's relaxation with 1/tau = 0 is
+// not that where a population is not finite.
 template <int MODE>
 __device__ __forceinline__ void step_remapped(const LbmDev &L, const typename Store<MODE>::T *__restrict__ fa,
                                               typename Store<MODE>::T *__restrict__ fb, CellVel<MODE> *cu,
@@ -498,7 +501,8 @@ __global__ void __launch_bounds__(256, LbmLaunch<MODE, NV>::blocks)
         C vx[NV], vy[NV], vz[NV];
         double pc[NV];
         if constexpr (MODE != 0 && NV == 2) {
-            // (an INFLOW cell does not relax; a fan's equilibrium replaces it)
+            // (an INFLOW cell does not relax; a fan's equilibrium replaces it,
+            // and one without a fan is in the remap list)
             const bool in0 = (fl & 3u) == CT_INFLOW, in1 = ((fl >> 8) & 3u) == CT_INFLOW;
             const float itau = (float)(1.0 / L.tau);
             float u0[3], u1[3], d0, d1;
@@ -793,8 +797,7 @@ __global__ void k_lbm_flags(const uint8_t *__restrict__ ct, int nx, int ny, int 
     }
 }
 
-// OUTFLOW cells that take their populations from another cell: the cell
-// type plus LF_REMAP, never LF_OPEN.
+// The cells of the remap list: the cell type plus LF_REMAP, never LF_OPEN.
 __global__ void k_lbm_remap_flags(const uint8_t *__restrict__ ct, const int *__restrict__ dst, int m,
                                   uint8_t *__restrict__ flags)
 {
@@ -993,6 +996,22 @@ void resolve_remap(const HostRoom &h, std::vector<int> &dst, std::vector<int> &s
     for (const auto &kv : moved) { dst.push_back(kv.first); src.push_back(kv.second); }
 }
 
+// Appends the INFLOW cells that no fan's box holds, each as its own source.
+void add_fanless_inflow(const HostRoom &h, std::vector<int> &dst, std::vector<int> &src)
+{
+    const int ny = h.g.ny, nz = h.g.nz;
+    const uint8_t *ct = h.ct.data(), *end = ct + h.g.n;
+    for (const uint8_t *p = ct; (p = static_cast<const uint8_t *>(memchr(p, CT_INFLOW, (size_t)(end - p)))); p++) {
+        const int c = (int)(p - ct), i = c / (ny * nz), j = c / nz % ny, k = c % nz;
+        bool fan = false;
+        for (const ffr_fan &f : h.fans)
+            fan = fan || (i >= f.i_min && i <= f.i_max && j >= f.j_min && j <= f.j_max && k >= f.k_min && k <= f.k_max);
+        if (fan) continue;
+        dst.push_back(c);
+        src.push_back(c);
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -1026,6 +1045,7 @@ int ffr_lbm_create(const ffr_room_desc *room, double tau, int max_steps, double 
         for (int c = 0; c < 3; c++) fan_lat[3 * f + c] = s->room.fans[f].vel[c] * p2l;
     std::vector<int> rd, rs;
     resolve_remap(s->room, rd, rs);
+    if (storage != FFR_LBM_FP64) add_fanless_inflow(s->room, rd, rs);
     const size_t es = storage == FFR_LBM_FP64 ? 8 : (storage == FFR_LBM_FP32 ? 4 : 2);
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t bytes = 2 * al(es * ftotal) + 4 * al(8 * g.n) + al(8 * g.nu) + al(8 * g.nv) +
