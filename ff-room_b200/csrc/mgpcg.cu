@@ -1490,13 +1490,6 @@ __global__ void __launch_bounds__(256) k_sp_restrict(PCGArgs A, const SplitState
     restrict_level(A, A.M.lv, l, gtid(), gthreads());
 }
 
-__global__ void __launch_bounds__(1024) k_sp_coarse(PCGArgs A, const SplitState *ss, int lo)
-{
-    chain_wait();
-    if (ss->done) return;
-    block_vcycle(A, lo);
-}
-
 __global__ void __launch_bounds__(kMidThreads, 1) k_sp_mid(PCGArgs A, const SplitState *ss, int mid)
 {
     chain_wait();
