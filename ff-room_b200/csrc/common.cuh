@@ -67,7 +67,7 @@ struct HostRoom {
     std::vector<ffr_fan> fans;
     std::vector<ffr_patch> patches;
     std::vector<ffr_heat_patch> heats;
-    long long n_fluid = 0;
+    long long n_fluid = 0, n_inflow = 0;
 };
 
 int load_room(const ffr_room_desc *d, HostRoom &out);

@@ -997,16 +997,24 @@ void resolve_remap(const HostRoom &h, std::vector<int> &dst, std::vector<int> &s
 }
 
 // Appends the INFLOW cells that no fan's box holds, each as its own source.
+// (The room is searched for them only where the boxes hold fewer INFLOW cells
+// than it has.)
 void add_fanless_inflow(const HostRoom &h, std::vector<int> &dst, std::vector<int> &src)
 {
-    const int ny = h.g.ny, nz = h.g.nz;
+    const int nx = h.g.nx, ny = h.g.ny, nz = h.g.nz;
     const uint8_t *ct = h.ct.data(), *end = ct + h.g.n;
+    std::vector<int> held;
+    for (const ffr_fan &f : h.fans)
+        for (int i = std::max(0, f.i_min); i <= std::min(nx - 1, f.i_max); i++)
+            for (int j = std::max(0, f.j_min); j <= std::min(ny - 1, f.j_max); j++)
+                for (int k = std::max(0, f.k_min); k <= std::min(nz - 1, f.k_max); k++)
+                    if (const int c = (i * ny + j) * nz + k; ct[c] == CT_INFLOW) held.push_back(c);
+    std::sort(held.begin(), held.end());
+    held.erase(std::unique(held.begin(), held.end()), held.end());
+    if ((long long)held.size() == h.n_inflow) return;
     for (const uint8_t *p = ct; (p = static_cast<const uint8_t *>(memchr(p, CT_INFLOW, (size_t)(end - p)))); p++) {
-        const int c = (int)(p - ct), i = c / (ny * nz), j = c / nz % ny, k = c % nz;
-        bool fan = false;
-        for (const ffr_fan &f : h.fans)
-            fan = fan || (i >= f.i_min && i <= f.i_max && j >= f.j_min && j <= f.j_max && k >= f.k_min && k <= f.k_max);
-        if (fan) continue;
+        const int c = (int)(p - ct);
+        if (std::binary_search(held.begin(), held.end(), c)) continue;
         dst.push_back(c);
         src.push_back(c);
     }

@@ -269,30 +269,33 @@ int load_room(const ffr_room_desc *d, HostRoom &r)
     for (double h : r.dxv) if (!(h > 0)) return fail(FFR_EINVAL, "non-positive x spacing");
     for (double h : r.dyv) if (!(h > 0)) return fail(FFR_EINVAL, "non-positive y spacing");
     for (double h : r.dzv) if (!(h > 0)) return fail(FFR_EINVAL, "non-positive z spacing");
-    // copy, range check and FLUID count in 256 k-cell pieces on all host threads
+    // copy, range check, FLUID and INFLOW counts in 256 k-cell pieces on all host threads
     r.ct.resize(n);
     const int pieces = (int)((n + (1 << 18) - 1) >> 18);
-    std::vector<long long> fluid(pieces, 0);
+    std::vector<long long> fluid(pieces, 0), inflow(pieces, 0);
     std::vector<char> bad(pieces, 0);
     parallel_slabs(pieces, [&](int p0, int p1) {
         for (int p = p0; p < p1; p++) {
             const long long b = (long long)p << 18, e = std::min(n, b + (1ll << 18));
             std::memcpy(r.ct.data() + b, d->cell_type + b, (size_t)(e - b));
-            long long f = 0;
+            long long f = 0, in = 0;
             uint8_t mx = 0;
             for (long long c = b; c < e; c++) {
                 const uint8_t t = r.ct[c];
                 f += (t == CT_FLUID);
+                in += (t == CT_INFLOW);
                 mx = std::max(mx, t);
             }
             fluid[p] = f;
+            inflow[p] = in;
             bad[p] = mx > CT_OUTFLOW;
         }
     });
-    r.n_fluid = 0;
+    r.n_fluid = r.n_inflow = 0;
     for (int p = 0; p < pieces; p++) {
         if (bad[p]) return fail(FFR_EINVAL, "cell_type value out of range");
         r.n_fluid += fluid[p];
+        r.n_inflow += inflow[p];
     }
     if (d->nfans < 0 || d->npatches < 0 || d->nheat < 0) return fail(FFR_EINVAL, "negative count");
     if (d->nfans > kMaxFans) return fail(FFR_ERANGE, "more than 120 fans");
