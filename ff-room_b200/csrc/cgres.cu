@@ -260,8 +260,9 @@ __device__ __noinline__ bool await_copies(int own, int plane2, int halo_bytes, u
 // Bound by the latency of an iteration's two reductions (about 900 cycles
 // each: staged values, one warp's tree per partial, st.async, mbarrier) and,
 // from K = 4 on, by shared-memory bandwidth (ten 8-byte accesses per cell).
-// Per iteration, k_cg before and this kernel: 6 000 cells 11.8 -> 2.7 us, 11.6 k
-// 12.2 -> 3.1, 25.7 k 12.1 -> 3.8, 50 k 13.1 -> 5.6.
+// Per iteration of a solve (slope over the iteration count), k_cg and this
+// kernel: 6 000 cells 11.6 and 1.8 us, 11.6 k 11.1 and 2.4, 25.7 k 11.9 and 3.4,
+// 50 k 12.4 and 5.2.
 //
 // Every wait is bounded.  A block whose wait runs out tells the others when
 // the cluster meets at the end, and then every copy still on its way is waited
@@ -481,10 +482,14 @@ __device__ __forceinline__ int chunk_of(int block, int v)
     return (block >> 4) * 32 + (block & 15) + 16 * (v >> 1) + 256 * (v & 1);
 }
 
-// Bound by the L2 round trips of the two exchanges (about 3 k cycles each of
-// 13 k per iteration).  Fences instead of numbered words cost 2-3 k cycles on
-// each side of an exchange.  Per iteration, k_cg before and this kernel: 72 k
-// cells 14.2 -> 6.7 us, 123 k 15.2 -> 6.9.
+// Bound by the two exchanges.  Of 13 k cycles per iteration at 123 k cells
+// (block 40, clock reads included) 4.4 k pass waiting for the block sums of
+// d.Ad, 4.2 k for those of r.r and the halo's words, 1.3 k go into forming and
+// publishing the sums, 0.9 k into the direction with its halo, 0.6 k into A d,
+// 0.5 k into the update of x and r, the rest into the final sums.  Fences instead
+// of numbered words cost 2-3 k cycles on each side of an exchange.  Per iteration
+// of a solve (slope over the iteration count), k_cg and this kernel: 72 k cells
+// 12.8 and 6.2 us, 123 k 15.2 and 6.3.
 //
 // ABSENT (self-test): the last block stays away from reduction A.absent_at.
 //

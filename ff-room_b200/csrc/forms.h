@@ -78,10 +78,10 @@ FFR_HD constexpr int cluster_blocks(int n, int K) { return (n + K * kResThreads 
 // follows the other in memory; placeable(K, blocks): the device holds a
 // cluster of `blocks` blocks of the form with K cells per thread.
 //
-// The smallest number of cells per thread that fits a cluster: the grid form
-// takes 6.8-7.0 us per iteration at any size, the cluster form 2.7 us at 6 k
-// cells to 5.9 us at 64 k, on 16 SMs instead of 128.  (Between the cluster
-// forms the order is not a measured one.)
+// The smallest number of cells per thread that fits a cluster.  Per iteration
+// with 1, 2, 4 and 8 cells per thread: 6 000 cells 1.8, 2.0, 2.7, 4.1 us;
+// 11.6 k -, 2.3, 3.0, 4.4; 25.7 k -, -, 3.2, 4.5; 50 k 5.0 with 8.  The grid form
+// takes 5.9 to 6.3 us at any size on 128 SMs instead of 16, k_cg 11 to 15 us.
 template <class Place>
 int cg_form(int nx, int ny, int nz, int smem, int sms, bool pair, Place placeable)
 {

@@ -432,10 +432,15 @@ __device__ __forceinline__ void step_remapped(const LbmDev &L, const typename St
 // Bound: memory, 2 x 19 populations, four cell values and a flag per cell, as
 // long as enough loads are in flight.  One cell per thread in the narrow modes
 // issued 19 loads of 2 or 4 bytes each and was bound by instructions (FP32 641
-// us and FP16 591 at 384 x 320 x 128, now 497 and 394; 306 and 188 at 301 x 203
-// x 101, now 217 and 183): pairs halve the memory instructions and the packed
-// FP32 arithmetic halves the collision.  Where the row is odd most directions
-// keep two loads, so odd rows gain less.  Waiting for the type of the source
+// us and FP16 591 at 384 x 320 x 128, now 497 and 394-412; 306 and 188 at 301 x
+// 203 x 101, now 217 and 183-189): pairs halve the memory instructions and the
+// packed FP32 arithmetic halves the collision.  Two loads are left for 10 of 19
+// directions with PAR 0, 12 with PAR 1, 6 with PAR 2.  That is not what decides:
+// of three lattices of 6.2 M cells FP16 takes 175 us with PAR 0 (302 x 202 x 102),
+// 196 with PAR 1 (301 x 202 x 101) and 189 with PAR 2 (301 x 203 x 101), FP32 210,
+// 221 and 217.  FP16 gains little from pairs at 5 to 6 M cells whatever the row
+// (240 x 200 x 100: 141 to 138); its bound there (3.2 TB/s) has not been found.
+// Waiting for the type of the source
 // cell before its population cost the rest (the masks come first instead, and
 // only cells next to a wall look at one), as did one load after another of the
 // re-mapped cells inside a warp of ordinary ones.
@@ -825,9 +830,9 @@ __global__ void k_lbm_fan_of(const uint8_t *__restrict__ ct, int nx, int ny, int
 // Checkpoint conversion between the stored populations and FP64 f in the
 // reference's layout f[q*N + c] (LBMSolver.hpp:77-82): FP64 storage holds f
 // itself, the narrow modes the shifted g = f - w_q.  SOLID cells stream
-// nothing and their slots of the second buffer are never written; they are
-// exported as 0, the value the reference's push streaming leaves in them
-// (LBMSolver.cpp:151-190), and never read by a step.
+// nothing and their slots hold arbitrary values (a step stores whatever it
+// formed there and uses none of it); they are exported as 0, the value the
+// reference's push streaming leaves in them (LBMSolver.cpp:151-190).
 template <int MODE>
 __global__ void k_lbm_export(int n, int np, const uint8_t *__restrict__ ct, const typename Store<MODE>::T *__restrict__ f,
                              double *__restrict__ out)

@@ -1968,8 +1968,9 @@ unsigned split_blocks_level0(long long n)
 // cells).  A large level takes two items per thread in blocks of 256, so each
 // block amortises its start-up; a level that cannot fill the GPU that way takes
 // one per thread in blocks of 128, which puts it on twice to four times as many
-// SMs (us per iteration: 315 k cells 112 -> 105, 1.0 M 159 -> 153, 7.9 M 522 -> 518;
-// with the line at 1.2 M cells instead of 400 k, 1.0 M 155).
+// SMs (us per iteration in a step graph, without and with: 307 k cells 107.7 and
+// 99.2, 590 k 125.8 and 121.3, 983 k 154.3 and 148.6, 2.0 M 215.8 and 209.3, 7.9 M
+// 518.5 and 513.6; with the line at 1.2 M cells, 1.0 M took 2 us more).
 constexpr long long kSmallLevelCells = 400000;
 struct LevelShape {
     unsigned blocks, threads;
